@@ -14,10 +14,7 @@
 
 #include "gnss_b200.h"
 #include "internal.h"
-#include "kernels.cuh"
-#include "zreg.cuh"
-#include "passreg.cuh"
-#include "passtc.cuh"
+#include "launch.h"
 #include "diag.cuh"
 
 using namespace gnss;
@@ -68,6 +65,11 @@ struct gnss_ctx {
     unsigned *d_err = nullptr;                    // [0] error word set by bounded waits that time out,
                                                   // [1] wait control (GNSS_OPT_TEST_WAIT; 0 normally)
     int test_wait = 0;                            // GNSS_OPT_TEST_WAIT
+    // tables of the dealiasing sphere for k_passd (set_bounds): largest kept |kx| per (kept ky, kz column) and
+    // largest kept |ky| per kz column, and the x passes' tiles that lie in the sphere
+    short *dtab_x = nullptr, *dtab_y = nullptr;
+    int *xlist = nullptr;
+    int n_xlist = 0;
     double2 *mean64 = nullptr;                    // FP32 contexts: FP64 mean-profile line (kx = kz = 0) of the
                                                   // state and history, [2][5][ny] (k_update)
     int nsm = 148;                                // SMs of the device
@@ -159,362 +161,7 @@ static inline int grid_for(long long n, int threads) {
     return (int)(b < cap ? (b < 1 ? 1 : b) : cap);
 }
 
-// Dynamic shared memory above 48 KB needs an opt-in, and the largest carveout
-// lets several blocks share an SM.
-template <class K> static cudaError_t prep_smem(K kern, int bytes) {
-    if (bytes > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (e != cudaSuccess) return e;
-    }
-    if (bytes > 0)
-        return cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                    (int)cudaSharedmemCarveoutMaxShared);
-    return cudaSuccess;
-}
-
-// ============================================================== per-size launchers
-template <class K> static int blocks_per_sm(K kern, int threads, int smem) {
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem) != cudaSuccess) {
-        cudaGetLastError();
-        n = 1;
-    }
-    return n < 1 ? 1 : n;
-}
-
-// Line lengths at which GNSS_VARIANT_AUTO takes the register kernels, as
-// measured on B200 (ensembles of 16 x 64^3 .. 2 x 192^3 and single jets at
-// 256^3, 512^3): the z kernel at every length it serves; the passes at
-// N = 96 .. 512 in FP32 (at N = 64 the staged pass: 8 931 against 7 759
-// Mpoint-steps/s for 16 x 64^3) and at N = 256, 512 in FP64 (below, staged:
-// 7 542 against 6 743 for 2 x 192^3).
-__host__ __device__ constexpr bool zr_auto_z(int n) { return zr_size(n); }
-__host__ __device__ constexpr bool zr_auto_pass(int n, bool fp64) {
-    return zr_size(n) && (fp64 ? n >= 256 : n != 64);
-}
-
-template <typename T> static const V2<T> *pass_twiddles(const PassPtrs<T> &, const void *tw) {
-    return reinterpret_cast<const V2<T> *>(tw);
-}
-
-// Launch of a kernel of the step.  Within a PdlScope that allows it, the
-// launch carries programmatic stream serialization: the kernel may start its
-// prologue on SMs the previous kernel in the stream has left and waits
-// (pdl_wait) before it touches the memory of the step.  Inside stream capture
-// the dependency becomes a programmatic graph edge.  Measured per step (FP32,
-// one scalar): 64^3 53.5 -> 40.9 us, 96^3 118.7 -> 107.3 us, 128^3 195.3 ->
-// 181.7 us, 192^3 579 -> 565 us.  Steps of more than 2^23 points launch
-// plainly: with programmatic launches the 256^3 and 512^3 FP64 steps measured
-// 0.5 - 2% slower.
-static thread_local bool t_pdl = false;
-struct PdlScope {
-    bool prev;
-    explicit PdlScope(bool on) : prev(t_pdl) { t_pdl = on; }
-    ~PdlScope() { t_pdl = prev; }
-};
-constexpr long long PDL_MAX_POINTS = 1LL << 23;
-template <typename... KA, typename... A>
-static cudaError_t launch_dep(void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cfg.attrs = at;
-    cfg.numAttrs = t_pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
-}
-
-// A persistent pass launch: one block per SM times the blocks that fit
-// (looked up once per kernel, from any host thread), at most one per work item.
-template <class K, class PP>
-static cudaError_t launch_persistent(K kern, std::atomic<int> &per_sm, int nt, int smem, int nsm, long long nitems,
-                                     cudaStream_t s, const PP &P, const PassSpec &sp, const void *tw,
-                                     unsigned *err = nullptr, bool with_err = false) {
-    cudaError_t e = prep_smem(kern, smem);
-    if (e != cudaSuccess) return e;
-    int ps = per_sm.load(std::memory_order_relaxed);
-    if (ps == 0) {
-        ps = blocks_per_sm(kern, nt, smem);
-        per_sm.store(ps, std::memory_order_relaxed);
-    }
-    long long grid = (long long)ps * nsm;
-    if (grid > nitems) grid = nitems;
-    if (with_err) {
-        if constexpr (std::is_invocable_v<K, PP, PassSpec, const float2 *, unsigned *>)
-            return launch_dep(kern, dim3((unsigned)grid), dim3(nt), smem, s, P, sp, reinterpret_cast<const float2 *>(tw),
-                              err);
-    } else {
-        if constexpr (!std::is_invocable_v<K, PP, PassSpec, const float2 *, unsigned *>)
-            return launch_dep(kern, dim3((unsigned)grid), dim3(nt), smem, s, P, sp, pass_twiddles(P, tw));
-    }
-    return cudaGetLastError();
-}
-
-template <typename T, int N> struct Launch {
-    // Members of a batch (sp.nmem > 1) run the MB instantiations, which exist for the register lengths
-    // (N = 64 .. 512); other lengths return cudaErrorNotSupported for a batch.
-    static cudaError_t pass(int sign, const PassPtrs<T> &P, const PassSpec &sp, const void *tw, int nsm,
-                            cudaStream_t s, int pvariant, unsigned *err) {
-        const bool mb = sp.nmem > 1;
-        const int ci = (sign < 0 ? 0 : 1) + (mb ? 2 : 0);   // occupancy cache index
-        if constexpr (sizeof(T) == 4 && ptc_size(N)) {
-            // split-TF32 DFT-GEMM transforms on the tensor cores (tiles of 8 columns)
-            if (pvariant == GNSS_VARIANT_TENSOR) {
-                using C = PTCfg<N>;
-                auto kern = mb ? (sign < 0 ? k_passtc<N, -1, true> : k_passtc<N, +1, true>)
-                               : (sign < 0 ? k_passtc<N, -1> : k_passtc<N, +1>);
-                static std::atomic<int> per_sm[4];
-                PassSpec s8 = sp;
-                const int cols = sp.ncols > sp.out_ncols ? sp.ncols : sp.out_ncols;
-                s8.ncolblk = (cols + C::NB - 1) / C::NB;
-                const long long nitems = (long long)s8.nmem * s8.nin * s8.outer.count() * s8.ncolblk;
-                return launch_persistent(kern, per_sm[ci], C::NT, C::SMEM, nsm, nitems, s,
-                                         reinterpret_cast<const PassPtrs<float> &>(P), s8, tw, err, true);
-            }
-        }
-        const long long nitems = (long long)sp.nmem * sp.nin * sp.outer.count() * sp.ncolblk;
-        if constexpr (zr_size(N)) {
-            // register-resident column transforms where they measured faster (512^3 FP32 step 7.34 against
-            // 8.39 ms, FP64 10.1 against 8.9 Gpoint-steps/s; 256^3 1.23 against 1.28 ms; N = 96 .. 192 with
-            // lane shuffles)
-            const bool reg = pvariant == GNSS_VARIANT_REGISTER ||
-                             ((pvariant == GNSS_VARIANT_AUTO || pvariant == GNSS_VARIANT_TENSOR) &&
-                              zr_auto_pass(N, sizeof(T) == 8));
-            if (reg) {
-                using C = PRCfg<T, N>;
-                auto kern = mb ? (sign < 0 ? k_passr<T, N, -1, true> : k_passr<T, N, +1, true>)
-                               : (sign < 0 ? k_passr<T, N, -1> : k_passr<T, N, +1>);
-                static std::atomic<int> per_sm[4];
-                return launch_persistent(kern, per_sm[ci], C::NT, C::SMEM, nsm, nitems, s, P, sp, tw);
-            }
-        }
-        using C = PassCfg<T, N>;
-        static std::atomic<int> per_sm[4];
-        if (mb) {
-            if constexpr (zr_size(N)) {
-                auto kern = sign < 0 ? k_pass<T, N, -1, true> : k_pass<T, N, +1, true>;
-                return launch_persistent(kern, per_sm[ci], C::NT, C::SMEM, nsm, nitems, s, P, sp, tw);
-            } else {
-                return cudaErrorNotSupported;
-            }
-        }
-        auto kern = sign < 0 ? k_pass<T, N, -1> : k_pass<T, N, +1>;
-        return launch_persistent(kern, per_sm[ci], C::NT, C::SMEM, nsm, nitems, s, P, sp, tw);
-    }
-    static cudaError_t zpass(int dir, const FieldSet<T> &f, int nfields, long long nlines, int nz2, T scale,
-                             const void *tw, cudaStream_t s) {
-        using C = ZCfg<T, N>;
-        long long npairs = (nlines + 1) / 2;
-        dim3 grid((unsigned)((npairs + ZWARPS - 1) / ZWARPS), (unsigned)nfields);
-        const V2<T> *t = reinterpret_cast<const V2<T> *>(tw);
-        auto kern = dir < 0 ? k_zpass<T, N, -1> : k_zpass<T, N, +1>;
-        cudaError_t e = prep_smem(kern, C::SMEM);
-        if (e != cudaSuccess) return e;
-        kern<<<grid, ZWARPS * 32, C::SMEM, s>>>(f, nlines, nz2, scale, t);
-        return cudaGetLastError();
-    }
-    template <int NPH, int NRAW, bool PP>
-    static cudaError_t zphys_k(const FieldSet<T> &f, const ZRecipeSet &zr, int nout, long long nlines, int ncp,
-                               int nkz, T scale, T alpha, double dkz, const void *tw, unsigned *err, int nsm,
-                               cudaStream_t s, int nmem, long long ms) {
-        if (nmem > 1) return cudaErrorNotSupported;   // batches run the register z kernel
-        using C = ZPCfg<T, N>;
-        const int pipe_b = C::pipe_bytes(NPH, NRAW, ncp, PP);
-        const int pipe = pipe_b <= C::SMEM_MAX ? 1 : 0;
-        const int smem = pipe ? pipe_b : C::work_bytes(NPH, PP);
-        auto kern = k_zphys<T, N, NPH, NRAW, PP>;
-        cudaError_t e = prep_smem(kern, smem);
-        if (e != cudaSuccess) return e;
-        int per_sm = blocks_per_sm(kern, NPH * 32, smem);
-        const long long mpairs = nlines / 2, npairs = mpairs * nmem;
-        long long grid = (long long)per_sm * nsm;
-        if (grid > npairs) grid = npairs;
-        return launch_dep(kern, dim3((unsigned)grid), dim3(NPH * 32), smem, s, f, zr, nout, npairs, ncp, nkz, pipe,
-                          scale, alpha, dkz, reinterpret_cast<const V2<T> *>(tw), err, mpairs, ms);
-    }
-    // ping-pong banks when they fit next to the staging area, else in place
-    template <int NPH, int NRAW>
-    static cudaError_t zphys_n(const FieldSet<T> &f, const ZRecipeSet &zr, int nout, long long nlines, int ncp,
-                               int nkz, T scale, T alpha, double dkz, const void *tw, unsigned *err, int nsm,
-                               cudaStream_t s, int nmem, long long ms) {
-        using C = ZPCfg<T, N>;
-        if (C::pipe_bytes(NPH, NRAW, ncp, true) <= C::SMEM_MAX)
-            return zphys_k<NPH, NRAW, true>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nmem,
-                                            ms);
-        return zphys_k<NPH, NRAW, false>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nmem, ms);
-    }
-    // register-resident line transforms (N = 64 .. 512, zr_size) when their shared memory fits
-    // diag != nullptr: the instantiation that also writes per-block vorticity sums there
-    template <int NPH, int NRAW>
-    static cudaError_t zreg_k(const FieldSet<T> &f, const ZRecipeSet &zr, int nout, long long nlines, int ncp, int nkz,
-                              T scale, T alpha, double dkz, const void *tw, unsigned *err, int nsm, cudaStream_t s,
-                              double *diag, int nmem, long long ms) {
-        if constexpr (zr_size(N)) {
-            const int smem = ZRCfg<T, N>::smem_bytes(NPH, NRAW, ncp);
-            if (smem > ZPCfg<T, N>::SMEM_MAX) return cudaErrorNotSupported;
-            auto kern = diag ? k_zreg<T, N, NPH, NRAW, true>
-                             : (nmem > 1 ? k_zreg<T, N, NPH, NRAW, false, true> : k_zreg<T, N, NPH, NRAW, false>);
-            cudaError_t e = prep_smem(kern, smem);
-            if (e != cudaSuccess) return e;
-            const int per_sm = blocks_per_sm(kern, NPH * 32, smem);
-            const long long mpairs = nlines / 2, npairs = mpairs * nmem;
-            long long grid = (long long)per_sm * nsm;
-            if (grid > npairs) grid = npairs;
-            if (diag && grid > STAT_BLOCKS) grid = STAT_BLOCKS;   // one row of sums per block
-            return launch_dep(kern, dim3((unsigned)grid), dim3(NPH * 32), smem, s, f, zr, nout, npairs, ncp, nkz, scale,
-                              alpha, dkz, reinterpret_cast<const V2<T> *>(tw), err, diag, mpairs, ms);
-        } else {
-            (void)f; (void)zr; (void)nout; (void)nlines; (void)ncp; (void)nkz; (void)scale; (void)alpha; (void)dkz;
-            (void)tw; (void)err; (void)nsm; (void)s; (void)diag; (void)nmem; (void)ms;
-            return cudaErrorNotSupported;
-        }
-    }
-    // warp-specialised register z kernel (N = 256, 512; FP32 with 9 quantities and 4 products, FP64 with 9 and 4
-    // or 12 and 5)
-    static constexpr bool zws_size() { return N == 256 || N == 512; }
-    template <int NPH, int NRAW>
-    static cudaError_t zws_kt(const FieldSet<T> &f, const ZRecipeSet &zr, int nout, long long nlines, int ncp,
-                              int nkz, T scale, T alpha, double dkz, const void *tw, unsigned *err, int nsm,
-                              cudaStream_t s, int nmem, long long ms) {
-        if (nmem > 1) return cudaErrorNotSupported;   // batches run the register z kernel
-        if constexpr (zws_size()) {
-            constexpr int NOUT = zws_nout<NPH>();
-            const int smem = ZRCfg<T, N>::smem_bytes_ws(NPH, NOUT, NRAW, ncp);
-            auto kern = k_zws<T, N, NPH, NRAW>;
-            cudaError_t e = prep_smem(kern, smem);
-            if (e != cudaSuccess) return e;
-            const int nt = (NPH + NOUT) * 32;
-            const int per_sm = blocks_per_sm(kern, nt, smem);
-            const long long mpairs = nlines / 2, npairs = mpairs * nmem;
-            long long grid = (long long)per_sm * nsm;
-            if (grid > npairs) grid = npairs;
-            return launch_dep(kern, dim3((unsigned)grid), dim3(nt), smem, s, f, zr, nout, npairs, ncp, nkz, scale, alpha,
-                              dkz, reinterpret_cast<const V2<T> *>(tw), err, mpairs, ms);
-        } else {
-            (void)f; (void)zr; (void)nout; (void)nlines; (void)ncp; (void)nkz; (void)scale; (void)alpha; (void)dkz;
-            (void)tw; (void)err; (void)nsm; (void)s; (void)nmem; (void)ms;
-            return cudaErrorNotSupported;
-        }
-    }
-    static cudaError_t zws_k(const FieldSet<T> &f, const ZRecipeSet &zr, int nph, int nraw, int nout, long long nlines,
-                             int ncp, int nkz, T scale, T alpha, double dkz, const void *tw, unsigned *err, int nsm,
-                             cudaStream_t s, int nmem, long long ms) {
-        if (nph == 9 && nraw == 10)
-            return zws_kt<9, 10>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nmem, ms);
-        if (nph == 12 && nraw == 13)
-            return zws_kt<12, 13>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nmem, ms);
-        return cudaErrorNotSupported;
-    }
-    static bool zws_fits(int nph, int nraw, int nout, int ncp) {
-        if constexpr (zws_size()) {
-            const bool fp32 = sizeof(T) == 4 && nph == 9 && nraw == 10 && nout == 4;
-            const bool fp64 = sizeof(T) == 8 && ((nph == 9 && nraw == 10 && nout == 4) ||
-                                                 (nph == 12 && nraw == 13 && nout == 5));
-            return (fp32 || fp64) && ZRCfg<T, N>::smem_bytes_ws(nph, nout, nraw, ncp) <= ZPCfg<T, N>::SMEM_MAX;
-        } else {
-            return false;
-        }
-    }
-    static bool zreg_fits(int nph, int nraw, int ncp) {
-        if constexpr (zr_size(N))
-            return ZRCfg<T, N>::smem_bytes(nph, nraw, ncp) <= ZPCfg<T, N>::SMEM_MAX;
-        else
-            return false;
-    }
-    // the z kernel a variant option selects: GNSS_VARIANT_WARPSPEC, _REGISTER or _STAGED
-    // AUTO: the warp-specialised kernel in FP64 where it fits (17 or 13 warps per SM against k_zreg's 12 or 9;
-    // measured at 512^3 with two scalars: z 6.18 -> 5.53 ms, one scalar 5.48 -> 4.59 ms; 256^3 0.95 -> 0.80 ms),
-    // the register kernel in FP32 (there k_zws measured slower: 2.52 -> 2.70 ms at 512^3)
-    static int zkernel(int zvariant, int nph, int nraw, int nout, int ncp) {
-        const bool ws = zvariant == GNSS_VARIANT_WARPSPEC || (zvariant == GNSS_VARIANT_AUTO && sizeof(T) == 8);
-        if (ws && zws_fits(nph, nraw, nout, ncp)) return GNSS_VARIANT_WARPSPEC;
-        const bool reg = zvariant == GNSS_VARIANT_REGISTER || zvariant == GNSS_VARIANT_WARPSPEC ||
-                         (zvariant == GNSS_VARIANT_AUTO && zr_auto_z(N));
-        return reg && zreg_fits(nph, nraw, ncp) ? GNSS_VARIANT_REGISTER : GNSS_VARIANT_STAGED;
-    }
-    // diag != nullptr: the register kernel with the fused vorticity sums (cudaErrorNotSupported where it does
-    // not exist)
-    static cudaError_t zphys(const FieldSet<T> &f, const ZRecipeSet &zr, int nph, int nraw, int nout,
-                             long long nlines, int ncp, int nkz, T scale, T alpha, double dkz, const void *tw,
-                             unsigned *err, int nsm, cudaStream_t s, int zvariant, double *diag = nullptr,
-                             int nmem = 1, long long ms = 0) {
-        if (diag) {
-            if (!zreg_fits(nph, nraw, ncp)) return cudaErrorNotSupported;
-            if (nph == 9 && nraw == 10)
-                return zreg_k<9, 10>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, diag, 1, 0);
-            if (nph == 12 && nraw == 13)
-                return zreg_k<12, 13>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, diag, 1, 0);
-            if (nph == 14 && nraw == 14)
-                return zreg_k<14, 14>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, diag, 1, 0);
-            return cudaErrorInvalidValue;
-        }
-        const int kern = zkernel(zvariant, nph, nraw, nout, ncp);
-        if (kern == GNSS_VARIANT_WARPSPEC)
-            return zws_k(f, zr, nph, nraw, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nmem, ms);
-        if (kern == GNSS_VARIANT_REGISTER) {
-            if (nph == 9 && nraw == 10)
-                return zreg_k<9, 10>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nullptr, nmem,
-                                     ms);
-            if (nph == 12 && nraw == 13)
-                return zreg_k<12, 13>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nullptr, nmem,
-                                      ms);
-            if (nph == 14 && nraw == 14)
-                return zreg_k<14, 14>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nullptr, nmem,
-                                      ms);
-            return cudaErrorInvalidValue;
-        }
-        if (nph == 9 && nraw == 10)
-            return zphys_n<9, 10>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nmem, ms);
-        if (nph == 12 && nraw == 13)
-            return zphys_n<12, 13>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nmem, ms);
-        if (nph == 14 && nraw == 14)
-            return zphys_n<14, 14>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nmem, ms);
-        return cudaErrorInvalidValue;
-    }
-};
-
-#define GNSS_SIZE_SWITCH(n, EXPR) GNSS_SIZE_SWITCH_OR(n, EXPR, return cudaErrorInvalidValue)
-#define GNSS_SIZE_SWITCH_OR(n, EXPR, DEFAULT)       \
-    switch (n) {                                    \
-        case 8: { constexpr int NN_ = 8; EXPR; }    \
-        case 12: { constexpr int NN_ = 12; EXPR; }  \
-        case 16: { constexpr int NN_ = 16; EXPR; }  \
-        case 24: { constexpr int NN_ = 24; EXPR; }  \
-        case 32: { constexpr int NN_ = 32; EXPR; }  \
-        case 48: { constexpr int NN_ = 48; EXPR; }  \
-        case 64: { constexpr int NN_ = 64; EXPR; }  \
-        case 96: { constexpr int NN_ = 96; EXPR; }  \
-        case 128: { constexpr int NN_ = 128; EXPR; } \
-        case 192: { constexpr int NN_ = 192; EXPR; } \
-        case 256: { constexpr int NN_ = 256; EXPR; } \
-        case 384: { constexpr int NN_ = 384; EXPR; } \
-        case 512: { constexpr int NN_ = 512; EXPR; } \
-        default: DEFAULT;                           \
-    }
-
-template <typename T>
-static cudaError_t launch_pass(int n, int sign, const PassPtrs<T> &P, const PassSpec &sp, const void *tw, int nsm,
-                               cudaStream_t s, int pvariant, unsigned *err) {
-    GNSS_SIZE_SWITCH(n, return (Launch<T, NN_>::pass(sign, P, sp, tw, nsm, s, pvariant, err)));
-}
-template <typename T>
-static cudaError_t launch_zpass(int n, int dir, const FieldSet<T> &f, int nfields, long long nlines, int nz2, T scale,
-                                const void *tw, cudaStream_t s) {
-    GNSS_SIZE_SWITCH(n, return (Launch<T, NN_>::zpass(dir, f, nfields, nlines, nz2, scale, tw, s)));
-}
-template <typename T>
-static cudaError_t launch_zphys(int n, const FieldSet<T> &f, const ZRecipeSet &zr, int nph, int nraw, int nout,
-                                long long nlines, int ncp, int nkz, T scale, T alpha, double dkz, const void *tw,
-                                unsigned *err, int nsm, cudaStream_t s, int zvariant, double *diag = nullptr,
-                                int nmem = 1, long long ms = 0) {
-    GNSS_SIZE_SWITCH(n, return (Launch<T, NN_>::zphys(f, zr, nph, nraw, nout, nlines, ncp, nkz, scale, alpha, dkz, tw,
-                                                      err, nsm, s, zvariant, diag, nmem, ms)));
-}
-
+// ============================================================== helpers
 template <typename T> static int pass_nb(int n) {
     switch (n) {
         case 8: return PassCfg<T, 8>::NB; case 12: return PassCfg<T, 12>::NB;
@@ -527,7 +174,6 @@ template <typename T> static int pass_nb(int n) {
     }
 }
 
-// ============================================================== helpers
 template <typename T> static V2<T> *fld(void *base, size_t nspec, int i) {
     return reinterpret_cast<V2<T> *>(base) + nspec * (size_t)i;
 }
@@ -744,6 +390,8 @@ static gnss_status nonlinear_and_update(gnss_ctx *c, const gnss_fields *state, v
         gnss_status st = ensure_scratch_step(c);
         if (st) return st;
     }
+    // both pass lengths on k_passd: the intermediates hold only what lies in the dealiasing sphere
+    const bool sphere = c->xlist && (c->pvariant == GNSS_VARIANT_AUTO || c->pvariant == GNSS_VARIANT_REGISTER);
     const PdlScope pdl((long long)g.nx * g.ny * g.nz <= PDL_MAX_POINTS);
     V2<T> *Pb = reinterpret_cast<V2<T> *>(bt.scratch ? bt.scratch : c->scratch);
     V2<T> *Qb = Pb + c->p_elems * (size_t)np;
@@ -785,6 +433,8 @@ static gnss_status nonlinear_and_update(gnss_ctx *c, const gnss_fields *state, v
             for (int v = 0; v < 2; ++v) { spx.vmul[i][v] = c->xvar_mul[i][v]; spx.vout[i][v] = c->xvar_out[i][v]; }
         }
         spx.nmem = bt.nmem; spx.ms_in = bt.ms_sh; spx.ms_out = bt.ms_scr;
+        spx.dtab = c->dtab_x; spx.dstride = c->ncp; spx.bound_in = 1;
+        if (sphere) { spx.list = c->xlist; spx.nlist = c->n_xlist; }
         CK(c, launch_pass<T>(g.nx, +1, P, spx, c->tw[0], c->nsm, s, c->pvariant, c->d_err));
     }
     {
@@ -798,6 +448,7 @@ static gnss_status nonlinear_and_update(gnss_ctx *c, const gnss_fields *state, v
             for (int v = 0; v < 2; ++v) { spy.vmul[i][v] = c->yvar_mul[i][v]; spy.vout[i][v] = c->yvar_out[i][v]; }
         }
         spy.nmem = bt.nmem; spy.ms_in = spy.ms_out = bt.ms_scr;
+        if (sphere) { spy.dtab = c->dtab_y; spy.bound_in = 1; }
         CK(c, launch_pass<T>(g.ny, +1, P, spy, c->tw[1], c->nsm, s, c->pvariant, c->d_err));
     }
     {
@@ -811,6 +462,7 @@ static gnss_status nonlinear_and_update(gnss_ctx *c, const gnss_fields *state, v
         for (int q = 0; q < nnl; ++q) { P.in[q] = Qf(q); P.out[q] = Pf(q); }
         PassSpec sp3 = step_spec<T>(c, Y_FWD_STEP, nnl);
         sp3.nmem = bt.nmem; sp3.ms_in = sp3.ms_out = bt.ms_scr;
+        if (sphere) { sp3.dtab = c->dtab_y; sp3.bound_out = 1; }
         CK(c, launch_pass<T>(g.ny, -1, P, sp3, c->tw[1], c->nsm, s, c->pvariant, c->d_err));
     }
     {
@@ -819,6 +471,10 @@ static gnss_status nonlinear_and_update(gnss_ctx *c, const gnss_fields *state, v
         for (int q = 0; q < nnl; ++q) { P.in[q] = Pf(q); P.out[q] = R.p[q]; }
         PassSpec sp4 = step_spec<T>(c, X_FWD_STEP, nnl);
         sp4.nmem = bt.nmem; sp4.ms_in = sp4.ms_out = bt.ms_scr;
+        if (sphere) {
+            sp4.dtab = c->dtab_x; sp4.dstride = c->ncp; sp4.bound_out = 1;
+            sp4.list = c->xlist; sp4.nlist = c->n_xlist;
+        }
         CK(c, launch_pass<T>(g.nx, -1, P, sp4, c->tw[0], c->nsm, s, c->pvariant, c->d_err));
     }
     {
@@ -1031,7 +687,7 @@ static gnss_status turb_stats_t(gnss_ctx *c, const gnss_fields *st, gnss_turb *o
 }
 
 template <typename T> static bool zdiag_fits(const gnss_ctx *c) {
-    GNSS_SIZE_SWITCH_OR(c->g.nz, return (Launch<T, NN_>::zreg_fits(c->n_phys, c->n_raw, c->ncp)), return false);
+    return zreg_available<T>(c->g.nz, c->n_phys, c->n_raw, c->ncp);
 }
 
 // One step with the calcTurbStats statistics of the state it starts from.  The
@@ -1133,9 +789,7 @@ gnss_status gnss_set_option(gnss_ctx *c, int key, int value) {
 }
 
 template <typename T> static int zkernel_of(const gnss_ctx *c) {
-    GNSS_SIZE_SWITCH_OR(c->g.nz,
-                        return (Launch<T, NN_>::zkernel(c->zvariant, c->n_phys, c->n_raw, c->nnl, c->ncp)),
-                        return GNSS_VARIANT_STAGED);
+    return zkernel_choice<T>(c->g.nz, c->zvariant, c->n_phys, c->n_raw, c->nnl, c->ncp);
 }
 
 gnss_status gnss_get_option(const gnss_ctx *c, int key, int *value) {
@@ -1350,6 +1004,63 @@ static void set_layout(gnss_ctx *c) {
     }
 }
 
+// Tables of the dealiasing sphere (one device allocation): the kept rows of a
+// column are those whose |index| does not exceed its bound, since k^2 grows
+// with the row's wavenumber; the bounds use the test k^2 > kmax^2 (solver.cu:36)
+// in the reference's order of evaluation.  With both pass lengths on k_passd
+// the x passes visit only the tiles (kept ky, column block) whose first column
+// has a mode inside the sphere, and the y passes leave the rows outside it
+// alone; x tiles are 128 bytes wide (8 FP64 or 16 FP32 columns).
+static gnss_status set_bounds(gnss_ctx *c) {
+    const Geom &g = c->g;
+    if (!pd_size(g.nx)) return GNSS_OK;
+    const int nky = c->ky_keep.count(), ncp = c->ncp, nb = c->elem == sizeof(double2) ? 8 : 16;
+    auto wn = [](int i, int n, double dk) { return (i < n / 2) ? dk * (double)i : dk * ((double)i - (double)n); };
+    auto ksq = [](double a, double b, double k) { return (a * a + b * b) + k * k; };
+    std::vector<short> t((size_t)(nky + 1) * ncp, (short)-1);
+    std::vector<int> list;
+    auto row = [&](short *r, double ko, int n, double dk) {   // bounds of one row of columns, falling with kz
+        int d = n / 2;
+        for (int z = 0; z < c->nkz; ++z) {
+            const double kc = wn(z, g.nz, g.dkz);
+            while (d >= 0 && ksq(dk * (double)d, ko, kc) > g.kmax2) --d;
+            r[z] = (short)d;
+        }
+    };
+    for (int y = 0; y < nky; ++y) {
+        short *r = t.data() + (size_t)y * ncp;
+        row(r, wn(c->ky_keep.expand(y), g.ny, g.dky), g.nx, g.dkx);
+        for (int b = 0; b < ncp / nb; ++b)
+            if (r[b * nb] >= 0) list.push_back(y << 8 | b);
+    }
+    {
+        short *r = t.data() + (size_t)nky * ncp;
+        int d = g.ny / 2;
+        for (int z = 0; z < c->nkz; ++z) {
+            while (d >= 0 && ksq(0.0, g.dky * (double)d, wn(z, g.nz, g.dkz)) > g.kmax2) --d;
+            r[z] = (short)d;
+        }
+    }
+    const size_t tb = (t.size() * sizeof(short) + 15) / 16 * 16, lb = list.size() * sizeof(int);
+    if (cudaMalloc(&c->dtab_x, tb + lb) != cudaSuccess) {
+        c->dtab_x = nullptr;
+        cudaGetLastError();
+        return GNSS_ERR_NOMEM;
+    }
+    c->owned_bytes += tb + lb;
+    if (cudaMemcpy(c->dtab_x, t.data(), t.size() * sizeof(short), cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(reinterpret_cast<char *>(c->dtab_x) + tb, list.data(), lb, cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaGetLastError();
+        return GNSS_ERR_CUDA;
+    }
+    if (pd_size(g.ny)) {
+        c->dtab_y = c->dtab_x + (size_t)nky * ncp;
+        c->xlist = reinterpret_cast<int *>(reinterpret_cast<char *>(c->dtab_x) + tb);
+        c->n_xlist = (int)list.size();
+    }
+    return GNSS_OK;
+}
+
 gnss_status gnss_create(const gnss_config *cfg, gnss_ctx **out) {
     if (!cfg || !out) return GNSS_ERR_INVALID;
     *out = nullptr;
@@ -1380,6 +1091,8 @@ gnss_status gnss_create(const gnss_config *cfg, gnss_ctx **out) {
     c->elem = k.precision == GNSS_FP64 ? sizeof(double2) : sizeof(float2);
     set_recipes(c);
     set_layout(c);
+    const gnss_status sb = set_bounds(c);
+    if (sb) { gnss_destroy(c); return sb; }
     const int ns[3] = {k.nx, k.ny, k.nz};
     for (int a = 0; a < 3; ++a) {
         c->tw[a] = k.precision == GNSS_FP64 ? make_twiddles<double>(ns[a], c) : make_twiddles<float>(ns[a], c);
@@ -1430,6 +1143,7 @@ gnss_status gnss_destroy(gnss_ctx *c) {
     if (c->turb_host) cudaFreeHost(c->turb_host);
     if (c->d_err) cudaFree(c->d_err);
     if (c->mean64) cudaFree(c->mean64);
+    if (c->dtab_x) cudaFree(c->dtab_x);
     if (c->res) cudaFree(c->res);
     if (c->run_sums) cudaFree(c->run_sums);
     if (c->run_sums_host) cudaFreeHost(c->run_sums_host);

@@ -21,6 +21,13 @@ namespace gnss {
 
 constexpr int MAXF = 16;
 
+// Line lengths the register transforms serve: N = 32 E with E = 8, 16 (one
+// transpose through shared memory, zr_fft) or E = 2, 3, 4, 6 (lane shuffles
+// only, zs_fft).
+__host__ __device__ constexpr bool zr_size(int n) {
+    return n == 64 || n == 96 || n == 128 || n == 192 || n == 256 || n == 512;
+}
+
 template <typename T> struct FieldSet { V2<T> *p[MAXF]; };
 
 struct Geom {
@@ -38,6 +45,11 @@ __device__ __forceinline__ double ksq3(double a, double b, double c) {
     return __dadd_rn(__dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)), __dmul_rn(c, c));
 }
 
+// Axis lengths k_passd (passd.cuh) serves.
+__host__ __device__ constexpr bool pd_size(int n) {
+    return n == 48 || n == 64 || n == 96 || n == 128 || n == 192 || n == 256 || n == 384 || n == 512;
+}
+
 // ------------------------------------------------------------ strided pass
 // A pass transforms along one axis of a field viewed as [outer][row][col]
 // (row = the transform index, col = the contiguous kz index).  Work items are
@@ -50,6 +62,9 @@ __device__ __forceinline__ double ksq3(double a, double b, double c) {
 // are known in the first, spectral-side pass).  Outputs are written with
 // their own strides (a transposed store for the x passes).
 enum : signed char { V_ONE = 0, V_IK_ROW = 1, V_IK_OUT = 2, V_IK_COL = 3, V_LAP = 4 };
+
+// |row index| of a transform row (the Nyquist row counts as N/2)
+template <int N> __device__ __forceinline__ int row_dist(int r) { return r <= N / 2 ? r : N - r; }
 
 // Kept indices of one axis under the spherical truncation: {0..K} and
 // {n-K..n-1}; K < 0 keeps every index.  Compact storage numbers the kept
@@ -85,6 +100,16 @@ struct PassSpec {
     signed char vout[MAXF][2]; // output field index of each output
     int nmem;                  // members of a batch (jets of one geometry in one launch), >= 1
     long long ms_in, ms_out;   // element strides between the members' inputs / outputs
+    // k_passd only
+    int in16, out16;           // rows of the source / destination start on 16-byte boundaries
+    const int *list;           // tiles visited, outer compact index << 8 | column block (null: all of them)
+    int nlist;
+    unsigned cb_magic;         // ceil(2^32 / ncolblk), 0 for one column block (tile index -> outer index)
+    // dtab[compact outer index * dstride + column]: the largest |row index| inside the dealiasing sphere, or -1
+    // (null: no bound).  Rows beyond a column's bound are not read (bound_in) or, beyond the bound of a tile's first
+    // column, not stored (bound_out).
+    const short *dtab;
+    int dstride, bound_in, bound_out;
 };
 template <typename T> struct PassPtrs {
     const V2<T> *in[MAXF];
@@ -885,7 +910,7 @@ k_stats_partial(FieldSet<T> st, int has_s, int has_c, Geom g, double *__restrict
         for (int q = 0; q < STAT_SUMS; ++q) partial[blockIdx.x * STAT_SUMS + q] = red[q][0];
 }
 
-__global__ void __launch_bounds__(STAT_SUMS * 32) k_stats_final(const double *__restrict__ partial, int nblocks,
+static __global__ void __launch_bounds__(STAT_SUMS * 32) k_stats_final(const double *__restrict__ partial, int nblocks,
                                                                  double *__restrict__ out) {
     // warp q sums column q: lanes stride the blocks, then a fixed shuffle tree
     pdl_wait();

@@ -45,7 +45,7 @@
 // the tile (A1, 16-byte stores) or, with the column and n2 % 4, the 32 words
 // of a row group's chunk (A3, 4-byte stores) hit distinct banks.
 #pragma once
-#include "passreg.cuh"
+#include "kernels.cuh"
 #include "tcgen05.cuh"
 
 #include <type_traits>

@@ -89,13 +89,6 @@ template <int S, typename V> struct Dft<16, S, V> {
     static __device__ __forceinline__ void run(V *v) { dft16<S>(v); }
 };
 
-// Line lengths the register transforms serve: N = 32 E with E = 8, 16 (one
-// transpose through shared memory, zr_fft) or E = 2, 3, 4, 6 (lane shuffles
-// only, zs_fft).
-__host__ __device__ constexpr bool zr_size(int n) {
-    return n == 64 || n == 96 || n == 128 || n == 192 || n == 256 || n == 512;
-}
-
 template <typename T, int N> struct ZRCfg {
     static_assert(zr_size(N), "register transforms serve N = 64, 96, 128, 192, 256, 512");
     static constexpr int E = N / 32;                    // elements per lane
