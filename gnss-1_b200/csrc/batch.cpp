@@ -397,7 +397,7 @@ gnss_status gnss_ensemble_autotune(gnss_ensemble *e, int steps, int *choices) {
     cudaEventCreate(&t0);
     cudaEventCreate(&t1);
     gnss_status st = GNSS_OK;
-    const int zvariants[3] = {GNSS_VARIANT_REGISTER, GNSS_VARIANT_STAGED, GNSS_VARIANT_WARPSPEC};
+    const int zvariants[2] = {GNSS_VARIANT_REGISTER, GNSS_VARIANT_STAGED};
     const int pvariants[3] = {GNSS_VARIANT_REGISTER, GNSS_VARIANT_STAGED, GNSS_VARIANT_TENSOR};
     std::vector<int> best(e->groups.size(), GNSS_VARIANT_AUTO);
     std::vector<bool> best_batched(e->groups.size(), false);
@@ -408,9 +408,9 @@ gnss_status gnss_ensemble_autotune(gnss_ensemble *e, int steps, int *choices) {
         float tbest = 0.f;
         int vbest = -1;
         bool bbest = false;
-        for (int combo = 0; combo < 18 && !st; ++combo) {
-            const int zv = zvariants[combo % 3], pv = pvariants[(combo / 3) % 3];
-            const bool batched = combo >= 9;   // the same kernels, as one batched launch per stage
+        for (int combo = 0; combo < 12 && !st; ++combo) {
+            const int zv = zvariants[combo % 2], pv = pvariants[(combo / 2) % 3];
+            const bool batched = combo >= 6;   // the same kernels, as one batched launch per stage
             if (pv == GNSS_VARIANT_TENSOR && !has_tensor_pass(m0.cfg)) continue;
             const int v = zv + 4 * pv;   // z variant + 4 * pass variant
             for (int i : g.members)
@@ -418,9 +418,6 @@ gnss_status gnss_ensemble_autotune(gnss_ensemble *e, int steps, int *choices) {
                     (st = gnss_set_option(e->m[i].ctx, GNSS_OPT_PVARIANT, pv)))
                     break;
             if (st) break;
-            int zk = 0;
-            if (zv == GNSS_VARIANT_WARPSPEC && (gnss_get_option(m0.ctx, GNSS_OPT_ZKERNEL, &zk) || zk != zv))
-                continue;   // no warp-specialised kernel here: the same kernels as the register choice
             if (batched && (g.members.size() < 2 || !gnss_batch_supported(m0.ctx))) continue;
             g.batched = batched;
             if ((st = fork_branches(e, ts)) || (st = group_step(e, g, 1)) || (st = join_branches(e, ts)))

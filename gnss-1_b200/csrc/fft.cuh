@@ -25,6 +25,19 @@ template <typename T> using V2 = typename Vec2<T>::type;
 
 template <typename V> __device__ __forceinline__ V cadd(V a, V b) { return V{a.x + b.x, a.y + b.y}; }
 template <typename V> __device__ __forceinline__ V csub(V a, V b) { return V{a.x - b.x, a.y - b.y}; }
+// FP32: real and imaginary part in one packed instruction (sm_100 f32x2)
+template <> __device__ __forceinline__ float2 cadd<float2>(float2 a, float2 b) {
+    float2 r;
+    asm("{\n\t.reg .b64 p, q, s;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tadd.rn.f32x2 s, p, q;\n\t"
+        "mov.b64 {%0, %1}, s;\n\t}" : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+template <> __device__ __forceinline__ float2 csub<float2>(float2 a, float2 b) {
+    float2 r;
+    asm("{\n\t.reg .b64 p, q, s;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tsub.rn.f32x2 s, p, q;\n\t"
+        "mov.b64 {%0, %1}, s;\n\t}" : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
 template <typename V> __device__ __forceinline__ V cmul(V a, V b) {
     return V{a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x};
 }

@@ -65,7 +65,7 @@ struct gnss_ctx {
     unsigned *d_err = nullptr;                    // [0] error word set by bounded waits that time out,
                                                   // [1] wait control (GNSS_OPT_TEST_WAIT; 0 normally)
     int test_wait = 0;                            // GNSS_OPT_TEST_WAIT
-    // tables of the dealiasing sphere for k_passd (set_bounds): largest kept |kx| per (kept ky, kz column) and
+    // tables of the dealiasing sphere for k_passd (make_tables, behind d_err): largest kept |kx| per (kept ky, kz column) and
     // largest kept |ky| per kz column, and the x passes' tiles that lie in the sphere
     short *dtab_x = nullptr, *dtab_y = nullptr;
     int *xlist = nullptr;
@@ -1004,59 +1004,61 @@ static void set_layout(gnss_ctx *c) {
     }
 }
 
-// Tables of the dealiasing sphere (one device allocation): the kept rows of a
-// column are those whose |index| does not exceed its bound, since k^2 grows
-// with the row's wavenumber; the bounds use the test k^2 > kmax^2 (solver.cu:36)
-// in the reference's order of evaluation.  With both pass lengths on k_passd
-// the x passes visit only the tiles (kept ky, column block) whose first column
-// has a mode inside the sphere, and the y passes leave the rows outside it
-// alone; x tiles are 128 bytes wide (8 FP64 or 16 FP32 columns).
-static gnss_status set_bounds(gnss_ctx *c) {
+// The error words and, behind them in the same allocation, the tables of the
+// dealiasing sphere for k_passd: the kept rows of a column are those whose
+// |index| does not exceed its bound, since k^2 grows with the row's
+// wavenumber; the bounds use the test k^2 > kmax^2 (solver.cu:36) in the
+// reference's order of evaluation.  With both pass lengths on k_passd the x
+// passes visit only the tiles (kept ky, column block) whose first column has a
+// mode inside the sphere, and the y passes leave the rows outside it alone; x
+// tiles are 128 bytes wide (8 FP64 or 16 FP32 columns).
+static gnss_status make_tables(gnss_ctx *c) {
     const Geom &g = c->g;
-    if (!pd_size(g.nx)) return GNSS_OK;
     const int nky = c->ky_keep.count(), ncp = c->ncp, nb = c->elem == sizeof(double2) ? 8 : 16;
     auto wn = [](int i, int n, double dk) { return (i < n / 2) ? dk * (double)i : dk * ((double)i - (double)n); };
     auto ksq = [](double a, double b, double k) { return (a * a + b * b) + k * k; };
-    std::vector<short> t((size_t)(nky + 1) * ncp, (short)-1);
+    std::vector<short> t;
     std::vector<int> list;
-    auto row = [&](short *r, double ko, int n, double dk) {   // bounds of one row of columns, falling with kz
-        int d = n / 2;
-        for (int z = 0; z < c->nkz; ++z) {
-            const double kc = wn(z, g.nz, g.dkz);
-            while (d >= 0 && ksq(dk * (double)d, ko, kc) > g.kmax2) --d;
-            r[z] = (short)d;
+    if (pd_size(g.nx)) {
+        t.assign((size_t)(nky + 1) * ncp, (short)-1);
+        for (int y = 0; y < nky; ++y) {   // largest kept |kx| of each (ky, kz) column; it falls with kz
+            short *r = t.data() + (size_t)y * ncp;
+            const double ko = wn(c->ky_keep.expand(y), g.ny, g.dky);
+            for (int z = 0, d = g.nx / 2; z < c->nkz; ++z) {
+                while (d >= 0 && ksq(g.dkx * (double)d, ko, wn(z, g.nz, g.dkz)) > g.kmax2) --d;
+                r[z] = (short)d;
+            }
+            for (int b = 0; b < ncp / nb; ++b)
+                if (r[b * nb] >= 0) list.push_back(y << 8 | b);
         }
-    };
-    for (int y = 0; y < nky; ++y) {
-        short *r = t.data() + (size_t)y * ncp;
-        row(r, wn(c->ky_keep.expand(y), g.ny, g.dky), g.nx, g.dkx);
-        for (int b = 0; b < ncp / nb; ++b)
-            if (r[b * nb] >= 0) list.push_back(y << 8 | b);
-    }
-    {
-        short *r = t.data() + (size_t)nky * ncp;
-        int d = g.ny / 2;
-        for (int z = 0; z < c->nkz; ++z) {
+        short *r = t.data() + (size_t)nky * ncp;   // largest kept |ky| of each kz column
+        for (int z = 0, d = g.ny / 2; z < c->nkz; ++z) {
             while (d >= 0 && ksq(0.0, g.dky * (double)d, wn(z, g.nz, g.dkz)) > g.kmax2) --d;
             r[z] = (short)d;
         }
     }
-    const size_t tb = (t.size() * sizeof(short) + 15) / 16 * 16, lb = list.size() * sizeof(int);
-    if (cudaMalloc(&c->dtab_x, tb + lb) != cudaSuccess) {
-        c->dtab_x = nullptr;
+    const size_t head = 256, tb = (t.size() * sizeof(short) + 15) / 16 * 16, lb = list.size() * sizeof(int);
+    std::vector<char> h(head + tb + lb, 0);
+    if (!t.empty()) memcpy(h.data() + head, t.data(), t.size() * sizeof(short));
+    if (!list.empty()) memcpy(h.data() + head + tb, list.data(), lb);
+    void *d = nullptr;
+    if (cudaMalloc(&d, h.size()) != cudaSuccess) {
         cudaGetLastError();
         return GNSS_ERR_NOMEM;
     }
+    c->d_err = static_cast<unsigned *>(d);
     c->owned_bytes += tb + lb;
-    if (cudaMemcpy(c->dtab_x, t.data(), t.size() * sizeof(short), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(reinterpret_cast<char *>(c->dtab_x) + tb, list.data(), lb, cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (cudaMemcpy(d, h.data(), h.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
         cudaGetLastError();
         return GNSS_ERR_CUDA;
     }
-    if (pd_size(g.ny)) {
-        c->dtab_y = c->dtab_x + (size_t)nky * ncp;
-        c->xlist = reinterpret_cast<int *>(reinterpret_cast<char *>(c->dtab_x) + tb);
-        c->n_xlist = (int)list.size();
+    if (!t.empty()) {
+        c->dtab_x = reinterpret_cast<short *>(static_cast<char *>(d) + head);
+        if (pd_size(g.ny)) {
+            c->dtab_y = c->dtab_x + (size_t)nky * ncp;
+            c->xlist = reinterpret_cast<int *>(static_cast<char *>(d) + head + tb);
+            c->n_xlist = (int)list.size();
+        }
     }
     return GNSS_OK;
 }
@@ -1091,8 +1093,8 @@ gnss_status gnss_create(const gnss_config *cfg, gnss_ctx **out) {
     c->elem = k.precision == GNSS_FP64 ? sizeof(double2) : sizeof(float2);
     set_recipes(c);
     set_layout(c);
-    const gnss_status sb = set_bounds(c);
-    if (sb) { gnss_destroy(c); return sb; }
+    const gnss_status tables = make_tables(c);
+    if (tables) { gnss_destroy(c); return tables; }
     const int ns[3] = {k.nx, k.ny, k.nz};
     for (int a = 0; a < 3; ++a) {
         c->tw[a] = k.precision == GNSS_FP64 ? make_twiddles<double>(ns[a], c) : make_twiddles<float>(ns[a], c);
@@ -1106,12 +1108,6 @@ gnss_status gnss_create(const gnss_config *cfg, gnss_ctx **out) {
         return GNSS_ERR_NOMEM;
     }
     c->owned_bytes += sizeof(double) * (STAT_BLOCKS * STAT_SUMS + STAT_SUMS);
-    if (cudaMalloc(&c->d_err, 2 * sizeof(unsigned)) != cudaSuccess ||
-        cudaMemset(c->d_err, 0, 2 * sizeof(unsigned)) != cudaSuccess) {
-        cudaGetLastError();
-        gnss_destroy(c);
-        return GNSS_ERR_NOMEM;
-    }
     if (k.precision == GNSS_FP32) {   // the mean-profile line in FP64 (k_update); zero: taken from the fields
         const size_t mb = sizeof(double2) * 10 * (size_t)k.ny;
         if (cudaMalloc(&c->mean64, mb) != cudaSuccess || cudaMemset(c->mean64, 0, mb) != cudaSuccess) {
@@ -1143,7 +1139,6 @@ gnss_status gnss_destroy(gnss_ctx *c) {
     if (c->turb_host) cudaFreeHost(c->turb_host);
     if (c->d_err) cudaFree(c->d_err);
     if (c->mean64) cudaFree(c->mean64);
-    if (c->dtab_x) cudaFree(c->dtab_x);
     if (c->res) cudaFree(c->res);
     if (c->run_sums) cudaFree(c->run_sums);
     if (c->run_sums_host) cudaFreeHost(c->run_sums_host);

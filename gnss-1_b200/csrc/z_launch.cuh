@@ -39,88 +39,87 @@ template <typename T, int N> struct ZLaunch {
                                             ms);
         return zphys_k<NPH, NRAW, false>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nmem, ms);
     }
-    // register-resident line transforms (N = 64 .. 512, zr_size) when their shared memory fits
-    // diag != nullptr: the instantiation that also writes per-block vorticity sums there
+    // FP32: k_zpipe, FP64: k_zws
+    template <int NPH> using ZBlock = std::conditional_t<sizeof(T) == 4, ZPipe<T, N, NPH>, ZWs<T, N, NPH>>;
+    // the register z kernels (N = 64 .. 512, zr_size); diag != nullptr: the instantiation that also writes per-block vorticity sums.
+    // Where the staged raw lines do not fit (FP64, N = 512: the colloid term, or a truncation that keeps more than
+    // 2/3 of the modes with two scalars) the warps read them from global memory.
+    template <int NPH, int NRAW, bool STAGED>
+    static cudaError_t zpipe_k(const FieldSet<T> &f, const ZRecipeSet &zr, long long nlines, int ncp, int nkz, T scale,
+                               T alpha, double dkz, const void *tw, unsigned *err, int nsm, cudaStream_t s, double *diag,
+                               int nmem, long long ms) {
+        using C = ZBlock<NPH>;
+        const int smem = C::smem_bytes(STAGED ? NRAW : 0, ncp);
+        auto pick = [&] {
+            if constexpr (sizeof(T) == 4)
+                return diag       ? k_zpipe<T, N, NPH, NRAW, true>
+                       : nmem > 1 ? k_zpipe<T, N, NPH, NRAW, false, true>
+                                  : k_zpipe<T, N, NPH, NRAW>;
+            else
+                return diag       ? k_zws<T, N, NPH, NRAW, true, false, STAGED>
+                       : nmem > 1 ? k_zws<T, N, NPH, NRAW, false, true, STAGED>
+                                  : k_zws<T, N, NPH, NRAW, false, false, STAGED>;
+        };
+        auto kern = pick();
+        cudaError_t e = prep_smem(kern, smem);
+        if (e != cudaSuccess) return e;
+        const int per_sm = blocks_per_sm(kern, C::NT, smem);
+        const long long mpairs = nlines / 2, npairs = mpairs * nmem;
+        long long grid = (long long)per_sm * nsm;
+        if (grid > npairs) grid = npairs;
+        if (diag && grid > STAT_BLOCKS) grid = STAT_BLOCKS;   // one row of sums per block
+        return launch_dep(kern, dim3((unsigned)grid), dim3(C::NT), smem, s, f, zr, npairs, ncp, nkz, scale, alpha, dkz,
+                          reinterpret_cast<const V2<T> *>(tw), err, diag, mpairs, ms);
+    }
     template <int NPH, int NRAW>
-    static cudaError_t zreg_k(const FieldSet<T> &f, const ZRecipeSet &zr, int nout, long long nlines, int ncp, int nkz,
-                              T scale, T alpha, double dkz, const void *tw, unsigned *err, int nsm, cudaStream_t s,
-                              double *diag, int nmem, long long ms) {
+    static cudaError_t zpipe_n(const FieldSet<T> &f, const ZRecipeSet &zr, long long nlines, int ncp, int nkz, T scale,
+                               T alpha, double dkz, const void *tw, unsigned *err, int nsm, cudaStream_t s, double *diag,
+                               int nmem, long long ms) {
         if constexpr (zr_size(N)) {
-            const int smem = ZRCfg<T, N>::smem_bytes(NPH, NRAW, ncp);
-            if (smem > ZPCfg<T, N>::SMEM_MAX) return cudaErrorNotSupported;
-            auto kern = diag ? k_zreg<T, N, NPH, NRAW, true>
-                             : (nmem > 1 ? k_zreg<T, N, NPH, NRAW, false, true> : k_zreg<T, N, NPH, NRAW, false>);
-            cudaError_t e = prep_smem(kern, smem);
-            if (e != cudaSuccess) return e;
-            const int per_sm = blocks_per_sm(kern, NPH * 32, smem);
-            const long long mpairs = nlines / 2, npairs = mpairs * nmem;
-            long long grid = (long long)per_sm * nsm;
-            if (grid > npairs) grid = npairs;
-            if (diag && grid > STAT_BLOCKS) grid = STAT_BLOCKS;   // one row of sums per block
-            return launch_dep(kern, dim3((unsigned)grid), dim3(NPH * 32), smem, s, f, zr, nout, npairs, ncp, nkz, scale,
-                              alpha, dkz, reinterpret_cast<const V2<T> *>(tw), err, diag, mpairs, ms);
-        } else {
-            (void)f; (void)zr; (void)nout; (void)nlines; (void)ncp; (void)nkz; (void)scale; (void)alpha; (void)dkz;
-            (void)tw; (void)err; (void)nsm; (void)s; (void)diag; (void)nmem; (void)ms;
-            return cudaErrorNotSupported;
+            if (ZBlock<NPH>::smem_bytes(NRAW, ncp) <= ZPCfg<T, N>::SMEM_MAX)
+                return zpipe_k<NPH, NRAW, true>(f, zr, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, diag, nmem, ms);
+            if constexpr (sizeof(T) == 8 && N == 512 && NPH > 9)
+                return zpipe_k<NPH, NRAW, false>(f, zr, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, diag, nmem, ms);
         }
-    }
-    // warp-specialised register z kernel (N = 256, 512; FP32 with 9 quantities and 4 products, FP64 with 9 and 4
-    // or 12 and 5)
-    static constexpr bool zws_size() { return N == 256 || N == 512; }
-    template <int NPH, int NRAW>
-    static cudaError_t zws_kt(const FieldSet<T> &f, const ZRecipeSet &zr, int nout, long long nlines, int ncp,
-                              int nkz, T scale, T alpha, double dkz, const void *tw, unsigned *err, int nsm,
-                              cudaStream_t s, int nmem, long long ms) {
-        if (nmem > 1) return cudaErrorNotSupported;   // batches run the register z kernel
-        if constexpr (zws_size()) {
-            constexpr int NOUT = zws_nout<NPH>();
-            const int smem = ZRCfg<T, N>::smem_bytes_ws(NPH, NOUT, NRAW, ncp);
-            auto kern = k_zws<T, N, NPH, NRAW>;
-            cudaError_t e = prep_smem(kern, smem);
-            if (e != cudaSuccess) return e;
-            const int nt = (NPH + NOUT) * 32;
-            const int per_sm = blocks_per_sm(kern, nt, smem);
-            const long long mpairs = nlines / 2, npairs = mpairs * nmem;
-            long long grid = (long long)per_sm * nsm;
-            if (grid > npairs) grid = npairs;
-            return launch_dep(kern, dim3((unsigned)grid), dim3(nt), smem, s, f, zr, nout, npairs, ncp, nkz, scale, alpha,
-                              dkz, reinterpret_cast<const V2<T> *>(tw), err, mpairs, ms);
-        } else {
-            (void)f; (void)zr; (void)nout; (void)nlines; (void)ncp; (void)nkz; (void)scale; (void)alpha; (void)dkz;
-            (void)tw; (void)err; (void)nsm; (void)s; (void)nmem; (void)ms;
-            return cudaErrorNotSupported;
-        }
-    }
-    static cudaError_t zws_k(const FieldSet<T> &f, const ZRecipeSet &zr, int nph, int nraw, int nout, long long nlines,
-                             int ncp, int nkz, T scale, T alpha, double dkz, const void *tw, unsigned *err, int nsm,
-                             cudaStream_t s, int nmem, long long ms) {
-        if (nph == 9 && nraw == 10)
-            return zws_kt<9, 10>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nmem, ms);
-        if (nph == 12 && nraw == 13)
-            return zws_kt<12, 13>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nmem, ms);
         return cudaErrorNotSupported;
     }
+    static cudaError_t zpipe(const FieldSet<T> &f, const ZRecipeSet &zr, int nph, int nraw, long long nlines, int ncp,
+                             int nkz, T scale, T alpha, double dkz, const void *tw, unsigned *err, int nsm,
+                             cudaStream_t s, double *diag, int nmem, long long ms) {
+        if (nph == 9 && nraw == 10)
+            return zpipe_n<9, 10>(f, zr, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, diag, nmem, ms);
+        if (nph == 12 && nraw == 13)
+            return zpipe_n<12, 13>(f, zr, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, diag, nmem, ms);
+        if (nph == 14 && nraw == 14)
+            return zpipe_n<14, 14>(f, zr, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, diag, nmem, ms);
+        return cudaErrorInvalidValue;
+    }
+    // the lines GNSS_VARIANT_WARPSPEC names (z length 256 or 512; FP32 with one scalar, FP64 with one or two,
+    // without the colloid term)
     static bool zws_fits(int nph, int nraw, int nout, int ncp) {
-        if constexpr (zws_size()) {
-            const bool fp32 = sizeof(T) == 4 && nph == 9 && nraw == 10 && nout == 4;
-            const bool fp64 = sizeof(T) == 8 && ((nph == 9 && nraw == 10 && nout == 4) ||
-                                                 (nph == 12 && nraw == 13 && nout == 5));
-            return (fp32 || fp64) && ZRCfg<T, N>::smem_bytes_ws(nph, nout, nraw, ncp) <= ZPCfg<T, N>::SMEM_MAX;
+        const bool fp32 = sizeof(T) == 4 && nph == 9 && nraw == 10 && nout == 4;
+        const bool fp64 = sizeof(T) == 8 && ((nph == 9 && nraw == 10 && nout == 4) ||
+                                             (nph == 12 && nraw == 13 && nout == 5));
+        if constexpr (N == 256 || N == 512) {
+            const int smem = nph == 9 ? ZBlock<9>::smem_bytes(nraw, ncp) : ZBlock<12>::smem_bytes(nraw, ncp);
+            return (fp32 || fp64) && smem <= ZPCfg<T, N>::SMEM_MAX;
         } else {
             return false;
         }
     }
     static bool zreg_fits(int nph, int nraw, int ncp) {
-        if constexpr (zr_size(N))
-            return ZRCfg<T, N>::smem_bytes(nph, nraw, ncp) <= ZPCfg<T, N>::SMEM_MAX;
-        else
+        if constexpr (zr_size(N)) {
+            if (sizeof(T) == 8 && N == 512 && nph > 9) return true;   // unstaged where the staging does not fit
+            const int smem = nph == 9    ? ZBlock<9>::smem_bytes(nraw, ncp)
+                             : nph == 12 ? ZBlock<12>::smem_bytes(nraw, ncp)
+                                         : ZBlock<14>::smem_bytes(nraw, ncp);
+            return smem <= ZPCfg<T, N>::SMEM_MAX;
+        } else {
             return false;
+        }
     }
-    // the z kernel a variant option selects: GNSS_VARIANT_WARPSPEC, _REGISTER or _STAGED
-    // AUTO: the warp-specialised kernel in FP64 where it fits (17 or 13 warps per SM against k_zreg's 12 or 9;
-    // measured at 512^3 with two scalars: z 6.18 -> 5.53 ms, one scalar 5.48 -> 4.59 ms; 256^3 0.95 -> 0.80 ms),
-    // the register kernel in FP32 (there k_zws measured slower: 2.52 -> 2.70 ms at 512^3)
+    // the z kernel a variant option selects: GNSS_VARIANT_WARPSPEC and _REGISTER both name k_zpipe (the first where
+    // zws_fits; AUTO reports it so in FP64), _STAGED k_zphys
     static int zkernel(int zvariant, int nph, int nraw, int nout, int ncp) {
         const bool ws = zvariant == GNSS_VARIANT_WARPSPEC || (zvariant == GNSS_VARIANT_AUTO && sizeof(T) == 8);
         if (ws && zws_fits(nph, nraw, nout, ncp)) return GNSS_VARIANT_WARPSPEC;
@@ -128,37 +127,13 @@ template <typename T, int N> struct ZLaunch {
                          (zvariant == GNSS_VARIANT_AUTO && zr_auto_z(N));
         return reg && zreg_fits(nph, nraw, ncp) ? GNSS_VARIANT_REGISTER : GNSS_VARIANT_STAGED;
     }
-    // diag != nullptr: the register kernel with the fused vorticity sums (cudaErrorNotSupported where it does
-    // not exist)
+    // diag != nullptr: k_zpipe with the fused vorticity sums (cudaErrorNotSupported where it does not exist)
     static cudaError_t zphys(const FieldSet<T> &f, const ZRecipeSet &zr, int nph, int nraw, int nout,
                              long long nlines, int ncp, int nkz, T scale, T alpha, double dkz, const void *tw,
                              unsigned *err, int nsm, cudaStream_t s, int zvariant, double *diag = nullptr,
                              int nmem = 1, long long ms = 0) {
-        if (diag) {
-            if (!zreg_fits(nph, nraw, ncp)) return cudaErrorNotSupported;
-            if (nph == 9 && nraw == 10)
-                return zreg_k<9, 10>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, diag, 1, 0);
-            if (nph == 12 && nraw == 13)
-                return zreg_k<12, 13>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, diag, 1, 0);
-            if (nph == 14 && nraw == 14)
-                return zreg_k<14, 14>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, diag, 1, 0);
-            return cudaErrorInvalidValue;
-        }
-        const int kern = zkernel(zvariant, nph, nraw, nout, ncp);
-        if (kern == GNSS_VARIANT_WARPSPEC)
-            return zws_k(f, zr, nph, nraw, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nmem, ms);
-        if (kern == GNSS_VARIANT_REGISTER) {
-            if (nph == 9 && nraw == 10)
-                return zreg_k<9, 10>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nullptr, nmem,
-                                     ms);
-            if (nph == 12 && nraw == 13)
-                return zreg_k<12, 13>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nullptr, nmem,
-                                      ms);
-            if (nph == 14 && nraw == 14)
-                return zreg_k<14, 14>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nullptr, nmem,
-                                      ms);
-            return cudaErrorInvalidValue;
-        }
+        if (diag || zkernel(zvariant, nph, nraw, nout, ncp) != GNSS_VARIANT_STAGED)
+            return zpipe(f, zr, nph, nraw, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, diag, nmem, ms);
         if (nph == 9 && nraw == 10)
             return zphys_n<9, 10>(f, zr, nout, nlines, ncp, nkz, scale, alpha, dkz, tw, err, nsm, s, nmem, ms);
         if (nph == 12 && nraw == 13)

@@ -13,13 +13,16 @@
 //   step B: E-point DFT in registers, twiddle W_32^(j k2'), and a G-point
 //           DFT across the lanes of a group with shuffles.
 // so a line crosses shared memory once per transform (instead of once per
-// radix-8 stage).  The C2R packing is done while loading the registers,
-// and the twiddles of step A are products of four table powers.  Each warp
-// leaves its physical quantity in its own scratch line, where the other warps
-// read it; the whole block forms the products in place, into the lines of the
-// forward warps.
+// radix-8 stage).  The C2R packing is done while loading the registers.  The
+// forward transform is the inverse one's flow graph reversed (zr_fft_rev), so
+// it takes the products where the inverse transforms leave their lines and
+// ends with the modes in order.  Two kernels use these pieces: k_zpipe (FP32)
+// and k_zws (FP64).
 #pragma once
 #include "kernels.cuh"
+#include "pk.cuh"
+
+#include <type_traits>
 
 namespace gnss {
 
@@ -95,20 +98,9 @@ template <typename T, int N> struct ZRCfg {
     static constexpr bool SHFL = E != 8 && E != 16;     // lane-shuffle scheme (no transpose)
     static constexpr int G = SHFL ? 1 : 32 / E;         // lanes per group in step B (transpose scheme)
     static constexpr int S = 32 + G;                    // transpose row stride (conflict-free both ways)
-    // table rows: in the FP32 passes the transpose scheme reads its step-A
-    // twiddles W_N^(lane k1) from the table (row k1 - 1, k1 = 1 .. E-1;
-    // TWFULL); the z kernels and FP64 build them from the powers
-    // W^(lane 2^b), b < LOGE (measured at 512^3 with the full table: FP32
-    // passes 0.06 ms faster per step, the z kernel 0.02 ms slower, FP64 0.1 ms
-    // slower); the shuffle scheme reads W_N^(lane k1), k1 = 1 .. E-1, then
-    // W_32^lane
-    static constexpr bool TWFULL = !SHFL && sizeof(T) == 4;
-    // rows of the table with (full, where TWFULL) or without the full step-A twiddles; the z kernels use the
-    // powers (their shared-memory traffic is the tighter limit), the passes the full table
-    __host__ __device__ static constexpr int rows(bool full) {
-        return (SHFL || (full && TWFULL)) ? E : (E == 16 ? 4 : 3);
-    }
-    static constexpr int LOGE = rows(false);
+    // table rows: the powers W_N^(lane 2^b), b < LOGE, of the transpose scheme's step-A twiddles; the shuffle scheme
+    // reads W_N^(lane k1), k1 = 1 .. E-1, then W_32^lane
+    static constexpr int LOGE = SHFL ? E : (E == 16 ? 4 : 3);
     // line padding.  Transpose scheme: a warp's stores of a transform's
     // output (zr_out_index: lane groups j = lane % G at E^2 sigma(j) apart,
     // lanes of a group on consecutive entries) take one wavefront per 128
@@ -128,19 +120,9 @@ template <typename T, int N> struct ZRCfg {
     static constexpr int SCR = SHFL ? PL : E * S;       // scratch line per warp (transposes, physical line)
     static_assert(SCR >= PL, "scratch holds a padded line");
     // index into the length-N table exp(-2 pi i j / N) of twiddle-table entry i
-    __host__ __device__ static constexpr int tw_index(int i, bool full = false) {
+    __host__ __device__ static constexpr int tw_index(int i) {
         const int row = i >> 5, l = i & 31;
-        return SHFL ? (row < E - 1 ? (l * (row + 1)) % N : (E * l) % N)
-                    : ((full && TWFULL) ? (l * (row + 1)) % N : (l << row) % N);
-    }
-    // twiddle powers, scratch lines (one per warp; they also hold the physical
-    // lines and the products), raw staging, mbarrier (16 B), kz table (ncp T)
-    __host__ __device__ static constexpr int smem_bytes(int nph, int nraw, int ncp) {
-        return (LOGE * 32 + nph * SCR + nraw * 2 * ncp) * (int)sizeof(V2<T>) + 16 + ncp * (int)sizeof(T);
-    }
-    // k_zws: one more scratch line per forward warp
-    __host__ __device__ static constexpr int smem_bytes_ws(int nph, int nout, int nraw, int ncp) {
-        return smem_bytes(nph + nout, nraw, ncp);
+        return SHFL ? (row < E - 1 ? (l * (row + 1)) % N : (E * l) % N) : (l << row) % N;
     }
 };
 
@@ -239,13 +221,45 @@ __device__ __forceinline__ void zs_fft(int lane, V2<T> *x, const V2<T> *tws) {
     }
 }
 
+// x[k1] *= W_N^(SIGN lane k1), the step-A twiddles of zr_fft (transpose scheme)
+template <typename T, int N, int SIGN> __device__ __forceinline__ void zr_twiddle(int lane, V2<T> *x, const V2<T> *tws) {
+    using V = V2<T>;
+    constexpr int E = ZRCfg<T, N>::E;
+    auto tw_at = [&](int b) {
+        V t = tws[32 * b + lane];
+        if (SIGN > 0) t.y = -t.y;
+        return t;
+    };
+    const V w1 = tw_at(0), w2 = tw_at(1), w4 = tw_at(2);
+    const V w3 = cmul(w1, w2);
+    if constexpr (E == 16) {
+        const V w8 = tw_at(3);
+        x[8] = cmul(x[8], w8);
+        x[9] = cmul(x[9], cmul(w1, w8));
+        x[10] = cmul(x[10], cmul(w2, w8));
+        x[11] = cmul(x[11], cmul(w3, w8));
+        x[12] = cmul(x[12], cmul(w4, w8));
+        x[13] = cmul(x[13], cmul(cmul(w1, w4), w8));
+        x[14] = cmul(x[14], cmul(cmul(w2, w4), w8));
+        x[15] = cmul(x[15], cmul(cmul(w3, w4), w8));
+    }
+    x[1] = cmul(x[1], w1);
+    x[2] = cmul(x[2], w2);
+    x[3] = cmul(x[3], w3);
+    x[4] = cmul(x[4], w4);
+    x[5] = cmul(x[5], cmul(w1, w4));
+    x[6] = cmul(x[6], cmul(w2, w4));
+    x[7] = cmul(x[7], cmul(w3, w4));
+}
+
 // Length-N DFT of one line held by a warp.  On entry x[m] is element
 // lane + 32 m; on return x[q] is element k1 + E q + E^2 zr_sigma(j) of the
 // transform, with k1 = lane / G, j = lane % G.  The one transpose goes
 // through scr at offsets at(k1, i) (row k1 = 0..E-1, entry i = 0..31);
-// tws: the twiddle table of ZRCfg (rows tw_index(., FULLTW)).
-template <typename T, int N, int SIGN, class AT = ZrScratch<T, N>, bool FULLTW = false>
-__device__ __forceinline__ void zr_fft(int lane, V2<T> *x, V2<T> *scr, const V2<T> *tws, AT at = AT{}) {
+// tws: the twiddle table of ZRCfg.
+template <typename T, int N, int SIGN>
+__device__ __forceinline__ void zr_fft(int lane, V2<T> *x, V2<T> *scr, const V2<T> *tws) {
+    const ZrScratch<T, N> at;
     using V = V2<T>;
     using Z = ZRCfg<T, N>;
     constexpr int E = Z::E, G = Z::G;
@@ -256,45 +270,7 @@ __device__ __forceinline__ void zr_fft(int lane, V2<T> *x, V2<T> *scr, const V2<
         return;
     } else {
     Dft<E, SIGN, V>::run(x);
-    {
-        if constexpr (Z::TWFULL && FULLTW) {   // every W^(lane k1) from the table
-#pragma unroll
-            for (int k1 = 1; k1 < E; ++k1) {
-                V t = tws[32 * (k1 - 1) + lane];
-                if (SIGN > 0) t.y = -t.y;
-                x[k1] = cmul(x[k1], t);
-            }
-        } else {
-            // W^k1 for k1 = 1, 2, 4 (, 8) from the table, the others as products
-            // (w3 = w1 w2, w5 = w1 w4, w6 = w2 w4, w7 = w3 w4, w(8+i) = w(i) w8),
-            // each applied as soon as it is formed
-            auto tw_at = [&](int b) {
-                V t = tws[32 * b + lane];
-                if (SIGN > 0) t.y = -t.y;
-                return t;
-            };
-            const V w1 = tw_at(0), w2 = tw_at(1), w4 = tw_at(2);
-            const V w3 = cmul(w1, w2);
-            if constexpr (E == 16) {
-                const V w8 = tw_at(3);
-                x[8] = cmul(x[8], w8);
-                x[9] = cmul(x[9], cmul(w1, w8));
-                x[10] = cmul(x[10], cmul(w2, w8));
-                x[11] = cmul(x[11], cmul(w3, w8));
-                x[12] = cmul(x[12], cmul(w4, w8));
-                x[13] = cmul(x[13], cmul(cmul(w1, w4), w8));
-                x[14] = cmul(x[14], cmul(cmul(w2, w4), w8));
-                x[15] = cmul(x[15], cmul(cmul(w3, w4), w8));
-            }
-            x[1] = cmul(x[1], w1);
-            x[2] = cmul(x[2], w2);
-            x[3] = cmul(x[3], w3);
-            x[4] = cmul(x[4], w4);
-            x[5] = cmul(x[5], cmul(w1, w4));
-            x[6] = cmul(x[6], cmul(w2, w4));
-            x[7] = cmul(x[7], cmul(w3, w4));
-        }
-    }
+    zr_twiddle<T, N, SIGN>(lane, x, tws);
 #pragma unroll
     for (int k1 = 0; k1 < E; ++k1) scr[at(k1, lane)] = x[k1];
     __syncwarp();
@@ -337,221 +313,341 @@ template <typename T, int N> __device__ __forceinline__ int zr_out_index(int lan
         return lane / Z::G + Z::E * q + Z::E * Z::E * zr_sigma<Z::G>(lane % Z::G);
 }
 
-// C2R packing (as pack_c2r_combo) straight into the registers of zr_fft:
-// x[m] = Z_n, n = lane + 32 m.  keep: bit m set when mode min(n, N - n) is a
-// kept kz mode (< nkz); tkz: kz wavenumbers (T) of the kept modes.
-template <typename T, int N>
-__device__ __forceinline__ void zr_pack(int lane, V2<T> *x, const ZRecipe rc, const V2<T> *a0, const V2<T> *a1,
-                                        int ncp, unsigned keep, const T *tkz) {
+// The reverse of zr_fft: on entry x[q] is element zr_out_index(lane, q), on
+// return x[m] is element lane + 32 m of the length-N DFT.  With input index
+// n = k1 + E k2 and output index k = l + 32 m, W_N^(n k) = W_E^(k1 m)
+// W_N^(k1 l) W_32^(k2 l): a 32-point DFT over k2 (k2 = q + E s, l = G l' + j:
+// a G-point DFT across the lanes, W_32^(q j), an E-point DFT over q), the
+// transpose, W_N^(k1 l) and an E-point DFT over k1.
+template <typename T, int N, int SIGN>
+__device__ __forceinline__ void zr_fft_rev(int lane, V2<T> *x, V2<T> *scr, const V2<T> *tws) {
     using V = V2<T>;
-    constexpr int E = ZRCfg<T, N>::E;
-    const bool any_kz = rc.ikz[0] || (a1 && rc.ikz[1]);
+    using Z = ZRCfg<T, N>;
+    constexpr int E = Z::E, G = Z::G;
+    if constexpr (Z::SHFL) {   // the 32-point DFT across lanes: bit-reversed input, decimation in time
+        (void)scr;
+        auto tw_at = [&](int i) {
+            V t = tws[i];
+            if (SIGN > 0) t.y = -t.y;
+            return t;
+        };
 #pragma unroll
-    for (int m = 0; m < E; ++m) {
-        const int n = lane + 32 * m;
-        const bool lo = 2 * n <= N;
-        const int k = lo ? n : N - n;
-        V z = V{T(0), T(0)};
-        if ((keep >> m) & 1u) {
-            const T kz = any_kz ? tkz[k] : T(0);
-            V a = a0[k], b = a0[ncp + k];
-            if (rc.ikz[0]) { a = V{-kz * a.y, kz * a.x}; b = V{-kz * b.y, kz * b.x}; }
-            if (rc.sgn[0] < 0) { a = V{-a.x, -a.y}; b = V{-b.x, -b.y}; }
-            if (a1) {
-                V c = a1[k], d = a1[ncp + k];
-                if (rc.ikz[1]) { c = V{-kz * c.y, kz * c.x}; d = V{-kz * d.y, kz * d.x}; }
-                if (rc.sgn[1] < 0) { a = csub(a, c); b = csub(b, d); }
-                else { a = cadd(a, c); b = cadd(b, d); }
-            }
-            if (k == 0 || 2 * k == N) { a.y = T(0); b.y = T(0); }
-            z = lo ? V{a.x - b.y, a.y + b.x} : V{a.x + b.y, b.x - a.y};
-        }
-        x[m] = z;
-    }
-}
-
-// The same packing with the recipe fixed at compile time, for the recipes the
-// step uses: sgn[0] = +1 and, with a second term, sgn[1] = -1 (IKZ0, IKZ1:
-// the kz factor on the first, second term; HAS1: a second term).  Same
-// arithmetic as zr_pack in the same order; the keep test is k < nkz, and
-// elements of which no lane is kept are skipped by a warp-uniform test.  The
-// imaginary parts are cleared only where they can be nonzero modes k = 0 and
-// k = N/2, i.e. lane 0 of elements 0 and E/2 (element E/2 uses the upper-half
-// formula at lane 0, which gives the same value once they are cleared).
-template <typename T, int N, bool IKZ0, bool HAS1, bool IKZ1>
-__device__ __forceinline__ void zr_pack_fixed(int lane, V2<T> *x, const V2<T> *a0, const V2<T> *a1, int ncp, int nkz,
-                                              const T *tkz) {
-    using V = V2<T>;
-    constexpr int E = ZRCfg<T, N>::E;
+        for (int h = 1; h <= 16; h <<= 1) {
+            const bool upper = (lane & h) != 0;
+            const T sg = upper ? T(-1) : T(1);
+            V w = V{T(1), T(0)};
+            if (h > 1 && upper) w = tw_at(32 * (E - 1) + (lane & (h - 1)) * (16 / h));
 #pragma unroll
-    for (int m = 0; m < E; ++m) {
-        const bool lo = m < E / 2;
-        const int kmin = lo ? 32 * m : N - 31 - 32 * m;   // smallest k of the element over the warp
-        V z = V{T(0), T(0)};
-        if (kmin < nkz) {
-            const int k = lo ? lane + 32 * m : N - lane - 32 * m;
-            if (k < nkz) {
-                V a = a0[k], b = a0[ncp + k];
-                T kz = T(0);
-                if constexpr (IKZ0 || IKZ1) kz = tkz[k];
-                if constexpr (IKZ0) { a = V{-kz * a.y, kz * a.x}; b = V{-kz * b.y, kz * b.x}; }
-                if constexpr (HAS1) {
-                    V c = a1[k], d = a1[ncp + k];
-                    if constexpr (IKZ1) { c = V{-kz * c.y, kz * c.x}; d = V{-kz * d.y, kz * d.x}; }
-                    a = csub(a, c);
-                    b = csub(b, d);
-                }
-                if (m == 0 || m == E / 2) {
-                    if (lane == 0) { a.y = T(0); b.y = T(0); }
-                }
-                z = lo ? V{a.x - b.y, a.y + b.x} : V{a.x + b.y, b.x - a.y};
+            for (int q = 0; q < E; ++q) {
+                const V t = h > 1 ? cmul(x[q], w) : x[q];
+                const V p = shfl_xor_v(t, h);
+                x[q] = V{p.x + sg * t.x, p.y + sg * t.y};
             }
         }
-        x[m] = z;
+#pragma unroll
+        for (int k1 = 1; k1 < E; ++k1) x[k1] = cmul(x[k1], tw_at(32 * (k1 - 1) + lane));
+    } else {
+        const int k1 = lane / G, j = lane % G;
+        if constexpr (G == 2) {
+            const T sg = j == 0 ? T(1) : T(-1);
+#pragma unroll
+            for (int q = 0; q < E; ++q) {
+                const V p = shfl_xor_v(x[q], 1);
+                x[q] = V{p.x + sg * x[q].x, p.y + sg * x[q].y};
+            }
+        } else {
+            const T s0 = (j & 1) ? T(-1) : T(1), s1 = (j & 2) ? T(-1) : T(1);
+#pragma unroll
+            for (int q = 0; q < E; ++q) {
+                const V p = shfl_xor_v(x[q], 1);
+                V c = V{p.x + s0 * x[q].x, p.y + s0 * x[q].y};
+                if (j == 3) c = mul_si<SIGN>(c);
+                const V p2 = shfl_xor_v(c, 2);
+                x[q] = V{p2.x + s1 * c.x, p2.y + s1 * c.y};
+            }
+        }
+        zr_tw32_all<SIGN, G, 1, E>(x, j);
+        Dft<E, SIGN, V>::run(x);
+        const ZrScratch<T, N> at;
+#pragma unroll
+        for (int l = 0; l < E; ++l) scr[at(k1, G * l + j)] = x[l];
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < E; ++k) x[k] = scr[at(k, lane)];
+        __syncwarp();
+        zr_twiddle<T, N, SIGN>(lane, x, tws);
+    }
+    Dft<E, SIGN, V>::run(x);
+}
+
+// C2R packing of one physical quantity (recipe rc: +-raw[r0] times (i kz)^ikz0, minus raw[r1] times (i kz)^ikz1
+// where there is a second term) into x[m] = Z_n, n = lane + 32 m: Z_k = A_k + i B_k and Z_{N-k} = conj A_k + i conj B_k
+// from the raw line pairs (line A: ncp values, then line B; the first nkz are the kept modes), the imaginary parts of
+// A, B at k = 0 and N/2 ignored.  Each kept mode is read once: element n's mirror N - n lies in lane 32 - l, element
+// E - 1 - m (lane 0: E - m), and gets there by shuffle.
+// FORM >= 0 fixes the recipe (bit 0: kz on the first term, bit 1: a second term, bit 2: kz on it), -1 tests it at run
+// time.  One copy for the plain lines and one for all others serve most kernels; a copy per recipe (FIXED) makes a
+// 13-warp block stall on instruction fetches (FP64, 512^3, one scalar: z 4.71 against 4.24 ms) but pays in the 17-warp
+// block with its 96 registers (two scalars: 5.10 against 5.58 ms).
+template <typename T, int N, int FORM>
+__device__ __forceinline__ void zl_pack_form(int lane, V2<T> *x, const ZRecipe rc, const V2<T> *a0, const V2<T> *a1,
+                                             int ncp, int nkz, const T *tkz) {
+    using V = V2<T>;
+    constexpr int E = N / 32, H = (E + 1) / 2;
+    const int mirror = (32 - lane) & 31;
+    const bool two = FORM < 0 ? rc.r[1] >= 0 : (FORM & 2) != 0, kz0 = FORM < 0 ? rc.ikz[0] != 0 : (FORM & 1) != 0;
+    const bool kz1 = FORM < 0 ? rc.ikz[1] != 0 : (FORM & 4) != 0;
+    auto mode = [&](int k, V &a, V &b) {
+        a = a0[k];
+        b = a0[ncp + k];
+        if (kz0) {
+            const T kz = tkz[k];
+            a = V{-kz * a.y, kz * a.x};
+            b = V{-kz * b.y, kz * b.x};
+        }
+        if (two) {
+            V c = a1[k], d = a1[ncp + k];
+            if (kz1) {
+                const T kz = tkz[k];
+                c = V{-kz * c.y, kz * c.x};
+                d = V{-kz * d.y, kz * d.x};
+            }
+            a = csub(a, c);
+            b = csub(b, d);
+        }
+    };
+#pragma unroll
+    for (int m = 0; m < E; ++m) x[m] = V{T(0), T(0)};
+#pragma unroll
+    for (int m = 0; m < H; ++m) {
+        if (32 * m >= nkz) continue;   // uniform: no kept mode in this element
+        const int k = lane + 32 * m;
+        V a = V{T(0), T(0)}, b = a;
+        if (k < nkz && 2 * k <= N) {
+            mode(k, a, b);
+            if ((m == 0 && lane == 0) || (E % 2 == 1 && 2 * k == N)) { a.y = T(0); b.y = T(0); }
+        }
+        const V lo = V{a.x - b.y, a.y + b.x}, hi = V{a.x + b.y, b.x - a.y};
+        const V in = V{__shfl_sync(0xffffffffu, hi.x, mirror), __shfl_sync(0xffffffffu, hi.y, mirror)};
+        if (m > 0 && lane == 0) x[E - m] = hi;
+        if (E % 2 == 1 && m == H - 1) {   // middle element: k <= N/2 in lanes 0 .. 16
+            x[m] = lane <= 16 ? lo : in;
+        } else {
+            x[m] = lo;
+            x[E - 1 - m] = lane == 0 ? V{T(0), T(0)} : in;
+        }
+    }
+    if (E % 2 == 0 && 2 * nkz > N) {   // lane 0 of element E/2 is the Nyquist mode
+        V a, b;
+        mode(N / 2, a, b);
+        if (lane == 0) x[E / 2] = V{a.x, b.x};
     }
 }
 
-// Recipe class for zr_pack_fixed (0 .. 5), or -1 for the general zr_pack.
-__device__ __forceinline__ int zr_kind(const ZRecipe &rc) {
-    if (rc.sgn[0] != 1) return -1;
-    if (rc.r[1] < 0) return rc.ikz[0] ? 1 : 0;
-    if (rc.sgn[1] != -1) return -1;
-    return 2 + (rc.ikz[0] ? 2 : 0) + (rc.ikz[1] ? 1 : 0);
+template <typename T, int N, bool FIXED = false>
+__device__ __forceinline__ void zl_pack(int lane, V2<T> *x, const ZRecipe rc, const V2<T> *a0, const V2<T> *a1, int ncp,
+                                        int nkz, const T *tkz) {
+    if constexpr (FIXED) {
+        const int form = (rc.ikz[0] ? 1 : 0) | (rc.r[1] >= 0 ? (rc.ikz[1] ? 6 : 2) : 0);
+        if (form == 0) zl_pack_form<T, N, 0>(lane, x, rc, a0, a1, ncp, nkz, tkz);
+        else if (form == 1) zl_pack_form<T, N, 1>(lane, x, rc, a0, a1, ncp, nkz, tkz);
+        else if (form == 2) zl_pack_form<T, N, 2>(lane, x, rc, a0, a1, ncp, nkz, tkz);
+        else if (form == 3) zl_pack_form<T, N, 3>(lane, x, rc, a0, a1, ncp, nkz, tkz);
+        else zl_pack_form<T, N, 6>(lane, x, rc, a0, a1, ncp, nkz, tkz);
+    } else if (rc.r[1] < 0 && !rc.ikz[0]) {
+        zl_pack_form<T, N, 0>(lane, x, rc, a0, a1, ncp, nkz, tkz);
+    } else {
+        zl_pack_form<T, N, -1>(lane, x, rc, a0, a1, ncp, nkz, tkz);
+    }
 }
 
-// Packs quantity `rc` of the staged raw line pairs into x (kind = zr_kind(rc)).
+// R2C unpacking of x[m] = Z_(lane + 32 m): A_k = (Z_k + conj Z_{N-k})/2, B_k = (Z_k - conj Z_{N-k})/(2i) of the kept
+// modes to the line pair at d (line A: ncp values, then line B; columns beyond N/2 are zero).
 template <typename T, int N>
-__device__ __forceinline__ void zr_pack_any(int kind, int lane, V2<T> *x, const ZRecipe rc, const V2<T> *raw, int rawf,
-                                            int ncp, int nkz, unsigned keep, const T *tkz) {
-    const V2<T> *a0 = raw + rc.r[0] * rawf;
-    const V2<T> *a1 = rc.r[1] >= 0 ? raw + rc.r[1] * rawf : nullptr;
-    switch (kind) {
-        case 0: zr_pack_fixed<T, N, false, false, false>(lane, x, a0, a1, ncp, nkz, tkz); break;
-        case 1: zr_pack_fixed<T, N, true, false, false>(lane, x, a0, a1, ncp, nkz, tkz); break;
-        case 2: zr_pack_fixed<T, N, false, true, false>(lane, x, a0, a1, ncp, nkz, tkz); break;
-        case 3: zr_pack_fixed<T, N, false, true, true>(lane, x, a0, a1, ncp, nkz, tkz); break;
-        case 4: zr_pack_fixed<T, N, true, true, false>(lane, x, a0, a1, ncp, nkz, tkz); break;
-        case 5: zr_pack_fixed<T, N, true, true, true>(lane, x, a0, a1, ncp, nkz, tkz); break;
-        default: zr_pack<T, N>(lane, x, rc, a0, a1, ncp, keep, tkz); break;
+__device__ __forceinline__ void zl_unpack(int lane, const V2<T> *x, V2<T> *d, int ncp) {
+    using V = V2<T>;
+    constexpr int E = N / 32;
+    const int mirror = (32 - lane) & 31;
+#pragma unroll
+    for (int m = 0; m <= E / 2; ++m) {
+        if (32 * m >= ncp) continue;   // uniform
+        const int k = lane + 32 * m;
+        const V s = lane == 0 ? x[(E - m) % E] : x[E - 1 - m];
+        const V zm = V{__shfl_sync(0xffffffffu, s.x, mirror), __shfl_sync(0xffffffffu, s.y, mirror)};
+        const V zk = x[m];
+        V A = V{T(0.5) * (zk.x + zm.x), T(0.5) * (zk.y - zm.y)};
+        V B = V{T(0.5) * (zk.y + zm.y), T(-0.5) * (zk.x - zm.x)};
+        if (2 * k > N) A = B = V{T(0), T(0)};
+        if (k < ncp) {
+            d[k] = A;
+            d[ncp + k] = B;
+        }
     }
+    for (int k = lane + 32 * (E / 2 + 1); k < ncp; k += 32) d[k] = d[ncp + k] = V{T(0), T(0)};   // padding of short lines
 }
 
-// Pointwise products of one line pair by the whole block: the physical
-// quantities are element pidx(n) of the lines `phys` (stride SCR), product f
-// goes to element pidx(n) of line f of `out` (stride SCR).  out may equal
-// phys (products in place over quantities 0 .. 4): each point is read in full
-// by one thread before that thread writes it, quantities 0 .. 4 are read
-// before any product is written, and products go to lines 0 .. 4 only.
-// Quantities: 0 u, 1 v, 2 w, 3 w1, 4 w2, 5 w3,
-// 6 sx, 7 sy, 8 sz, [9 cx, 10 cy, 11 cz], [12 c, 13 lap s]; products as
-// zphys_products: (w x u) (crossProductKernel_mgpu, solver.cu:139-164),
-// u . grad s (dotKernel_mgpu, solver.cu:342-356) and the colloid term
-// (colloidAdvectionKernel_mgpu, solver.cu:374-388).
-// With DIAG, the thread also adds to acc the vorticity sums of its points
-// (ZR_VORT_SUMS: |w|, w_x^2, w_y^2, w_z^2, both lines of the pair), the sums
-// of k_vort_partial (statistics.cu:1211-1305), from the physical quantities 3,
-// 4, 5 = w_x, w_y, w_z it reads anyway.
+// elementwise products of two real lines (x, y)
+__device__ __forceinline__ float2 lmul(float2 a, float2 b) {
+    float2 o;
+    f2_get(f2(a.x, a.y) * f2(b.x, b.y), o.x, o.y);
+    return o;
+}
+__device__ __forceinline__ double2 lmul(double2 a, double2 b) { return double2{a.x * b.x, a.y * b.y}; }
+__device__ __forceinline__ float2 lfma(float2 a, float2 b, float2 c) {
+    float2 o;
+    f2_get(pfma(f2(a.x, a.y), f2(b.x, b.y), f2(c.x, c.y)), o.x, o.y);
+    return o;
+}
+__device__ __forceinline__ double2 lfma(double2 a, double2 b, double2 c) {
+    return double2{a.x * b.x + c.x, a.y * b.y + c.y};
+}
+template <typename V> __device__ __forceinline__ V lneg(V a) { return V{-a.x, -a.y}; }
+// and of one
+__device__ __forceinline__ double lmul(double a, double b) { return a * b; }
+__device__ __forceinline__ double lfma(double a, double b, double c) { return a * b + c; }
+template <> __device__ __forceinline__ double lneg<double>(double a) { return -a; }
+
+// Physical lines and their products.  A warp leaves a physical line in shared
+// memory where its transform ends: element zr_out_index(lane, q) at
+// zl_base(lane) + q zl_stride() of the line (PADB / PADC padding: no bank
+// conflicts), and the forward warps read the products' factors at the same
+// places.  Quantities: 0 u, 1 v, 2 w, 3 w1, 4 w2, 5 w3, 6 sx, 7 sy, 8 sz,
+// [9 cx, 10 cy, 11 cz], [12 c, 13 lap s].
+template <typename T, int N> __device__ __forceinline__ int zl_base(int lane) {
+    using Z = ZRCfg<T, N>;
+    if constexpr (Z::SHFL)
+        return (Z::E + Z::PADC) * (int)(__brev((unsigned)lane) >> 27);
+    else
+        return lane / Z::G + (Z::E * Z::E + Z::PADP) * zr_sigma<Z::G>(lane % Z::G);
+}
+template <typename T, int N> __host__ __device__ constexpr int zl_stride() {
+    return ZRCfg<T, N>::SHFL ? 1 : ZRCfg<T, N>::E;
+}
+// The inverse transforms leave the lines unscaled; their 1/N^3 enters as
+// scale^2 on u, v, w (one factor of every product), except with the colloid
+// term, whose products have none of them: there every line is scaled.
+template <int NPH> __host__ __device__ constexpr bool zr_fold_scale() { return NPH < 14; }
+template <typename T, int NPH> __device__ __forceinline__ T zr_line_scale(int q, T scale) {
+    return zr_fold_scale<NPH>() ? (q < 3 ? scale * scale : T(1)) : scale;
+}
+// Product f at this lane's points: (w x u)_f (crossProductKernel_mgpu,
+// solver.cu:139-164) for f < 3, u . grad s (dotKernel_mgpu, solver.cu:342-356)
+// for 3, u . grad c and the colloid term (colloidAdvectionKernel_mgpu,
+// solver.cu:374-388) for 4.  With DIAG the warp of product 0 also adds the
+// vorticity sums of its points to acc (ZR_VORT_SUMS: |w|, w_x^2, w_y^2, w_z^2,
+// both lines; statistics.cu:1211-1305).
 constexpr int ZR_VORT_SUMS = 4;
-template <typename T, int N, int NPH, bool DIAG = false>
-__device__ __forceinline__ void zr_products(const V2<T> *phys, V2<T> *out, T alpha, double *acc = nullptr) {
+template <typename T, int N, int NPH, bool DIAG>
+__device__ __forceinline__ void zl_product(int f, int lane, V2<T> *x, const V2<T> *lines, T alpha, T scale, double *acc) {
     using V = V2<T>;
     using Z = ZRCfg<T, N>;
-    constexpr int SCR = Z::SCR;
-    constexpr bool has_c = NPH >= 12, has_al = NPH >= 14;
-    for (int n = threadIdx.x; n < N; n += blockDim.x) {
-        const int pn = Z::pidx(n);
-        const V *p = phys + pn;
-        const V u = p[0 * SCR], v = p[1 * SCR], w = p[2 * SCR];
-        const V o1 = p[3 * SCR], o2 = p[4 * SCR], o3 = p[5 * SCR];
-        const V sx = p[6 * SCR], sy = p[7 * SCR], sz = p[8 * SCR];
+    constexpr int E = Z::E, ST = zl_stride<T, N>(), L = Z::SCR;
+    const V *p = lines + zl_base<T, N>(lane);
+    if (f < 3) {
+        // w2 w - w3 v, w3 u - w1 w, w1 v - w2 u
+        const V *a = p + (f == 2 ? 3 : f + 4) * L, *b = p + (f == 0 ? 2 : f - 1) * L;
+        const V *c = p + (f == 0 ? 5 : f + 2) * L, *d = p + (f == 0 ? 1 : f == 1 ? 2 : 0) * L;
+#pragma unroll
+        for (int q = 0; q < E; ++q) x[q] = lfma(a[q * ST], b[q * ST], lneg(lmul(c[q * ST], d[q * ST])));
         if constexpr (DIAG) {
-            const double ax = o1.x, ay = o2.x, az = o3.x, bx = o1.y, by = o2.y, bz = o3.y;
-            acc[0] += sqrt(ax * ax + ay * ay + az * az) + sqrt(bx * bx + by * by + bz * bz);
-            acc[1] += ax * ax + bx * bx;
-            acc[2] += ay * ay + by * by;
-            acc[3] += az * az + bz * bz;
+            if (f == 0) {
+                const double s = zr_fold_scale<NPH>() ? (double)scale : 1.0;
+#pragma unroll
+                for (int q = 0; q < E; ++q) {
+                    const V w1 = p[3 * L + q * ST], w2 = p[4 * L + q * ST], w3 = p[5 * L + q * ST];
+                    const double ax = s * w1.x, ay = s * w2.x, az = s * w3.x, bx = s * w1.y, by = s * w2.y, bz = s * w3.y;
+                    acc[0] += sqrt(ax * ax + ay * ay + az * az) + sqrt(bx * bx + by * by + bz * bz);
+                    acc[1] += ax * ax + bx * bx;
+                    acc[2] += ay * ay + by * by;
+                    acc[3] += az * az + bz * bz;
+                }
+            }
         }
-        V *o = out + pn;
-        o[0 * SCR] = V{o2.x * w.x - o3.x * v.x, o2.y * w.y - o3.y * v.y};
-        o[1 * SCR] = V{-o1.x * w.x + o3.x * u.x, -o1.y * w.y + o3.y * u.y};
-        o[2 * SCR] = V{o1.x * v.x - o2.x * u.x, o1.y * v.y - o2.y * u.y};
-        o[3 * SCR] = V{u.x * sx.x + v.x * sy.x + w.x * sz.x, u.y * sx.y + v.y * sy.y + w.y * sz.y};
-        if constexpr (has_c) {
-            const V cx = p[9 * SCR], cy = p[10 * SCR], cz = p[11 * SCR];
-            const V adv = V{u.x * cx.x + v.x * cy.x + w.x * cz.x, u.y * cx.y + v.y * cy.y + w.y * cz.y};
-            if constexpr (has_al) {
-                const V cc = p[12 * SCR], ls = p[13 * SCR];
-                const V dr = V{ls.x * cc.x + cx.x * sx.x + cy.x * sy.x + cz.x * sz.x,
-                               ls.y * cc.y + cx.y * sx.y + cy.y * sy.y + cz.y * sz.y};
-                o[4 * SCR] = V{alpha * dr.x + adv.x, alpha * dr.y + adv.y};
-            } else {
-                o[4 * SCR] = adv;
+    } else {
+        const V *g = p + (f == 3 ? 6 : 9) * L;
+#pragma unroll
+        for (int q = 0; q < E; ++q)
+            x[q] = lfma(p[2 * L + q * ST], g[2 * L + q * ST],
+                        lfma(p[L + q * ST], g[L + q * ST], lmul(p[q * ST], g[q * ST])));
+        if constexpr (NPH >= 14) {
+            if (f == 4) {
+                const V al = V{alpha, alpha};
+#pragma unroll
+                for (int q = 0; q < E; ++q) {
+                    const V *h = p + q * ST;
+                    V dr = lmul(h[13 * L], h[12 * L]);
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) dr = lfma(h[(9 + i) * L], h[(6 + i) * L], dr);
+                    x[q] = lfma(al, dr, x[q]);
+                }
             }
         }
     }
 }
 
-// R2C output of one product line: the length-N transform in x (element
-// zr_out_index(lane, q) in x[q]) goes through the warp's scratch line, and the
-// kept modes of the two real lines of the pair are stored as the raw layout
-// ([A: ncp][B: ncp]) at d.
-template <typename T, int N>
-__device__ __forceinline__ void zr_store_r2c(int lane, const V2<T> *x, V2<T> *scr, V2<T> *d, int ncp) {
-    using V = V2<T>;
+// Shared memory and block shape of k_zpipe: one physical line per inverse
+// warp (its transposes run in it, too), transpose scratch per forward warp
+// (lengths with a transpose), the staged raw line pairs, an mbarrier, the kz
+// table.
+template <int NPH> __host__ __device__ constexpr int z_nout() { return NPH >= 12 ? 5 : 4; }
+template <typename T, int N, int NPH> struct ZPipe {   // FP32
     using Z = ZRCfg<T, N>;
-#pragma unroll
-    for (int q = 0; q < Z::E; ++q) scr[Z::pidx(zr_out_index<T, N>(lane, q))] = x[q];
-    __syncwarp();
-    for (int k = lane; k < ncp; k += 32) {
-        V A = V{T(0), T(0)}, B = V{T(0), T(0)};
-        if (2 * k <= N) {
-            const V zk = scr[Z::pidx(k)];
-            const V zm = scr[Z::pidx((N - k) % N)];
-            A = V{T(0.5) * (zk.x + zm.x), T(0.5) * (zk.y - zm.y)};
-            B = V{T(0.5) * (zk.y + zm.y), T(-0.5) * (zk.x - zm.x)};
-        }
-        d[k] = A;
-        d[ncp + k] = B;
+    static constexpr int NOUT = z_nout<NPH>(), NT = (NPH + NOUT) * 32;
+    static constexpr int LINE = Z::SCR;
+    static constexpr int FSCR = Z::SHFL ? 0 : Z::SCR;
+    // blocks per SM the registers are sized for
+    static constexpr int MINB = NPH <= 9 ? (N <= 192 ? 3 : 2) : NPH == 12 || N <= 192 ? 2 : 1;
+    __host__ __device__ static constexpr int smem_bytes(int nraw, int ncp) {
+        return (Z::LOGE * 32 + NPH * LINE + NOUT * FSCR + nraw * 2 * ncp) * (int)sizeof(V2<T>) + 16 + ncp * (int)sizeof(T);
     }
-    __syncwarp();   // scratch reused by the next transform
-}
+};
 
-// Persistent: block b handles line pairs b, b + gridDim.x, ... of all members
-// of a batch (npairs in all, mpairs per member, members ms elements apart);
-// warp q forms physical quantity q.  The raw lines of the next pair arrive by
-// cp.async.bulk (CTA-local, no multicast) while the current pair is
-// processed; a wait that times out sets bit 0 of *err and the block stops.
-// With DIAG the block also writes one row of ZR_VORT_SUMS vorticity sums over
-// its points to diag[blockIdx.x] (fixed-order reduction), for the statistics
-// of the state the step starts from.
+// The fused z stage in FP32 as a pipeline over line pairs, NPH inverse and NOUT
+// forward warps per block; block b handles line pairs b, b + gridDim.x, ... of
+// all members of a batch (npairs in all, mpairs per member, members ms
+// elements apart).  Between two block barriers,
+//   A  the inverse warps pack pair p + 1 (registers) while the forward warps
+//      read pair p's physical lines and form its products (registers);
+//   B  the inverse warps transform p + 1 and leave its physical lines while
+//      the forward warps transform p's products and store them over raw
+//      fields 0 .. NOUT-1 of the pair.
+// Every warp carries one line in registers and the products never pass through
+// shared memory.  The raw lines of the pair after the next arrive by
+// cp.async.bulk (CTA-local, no multicast) during B; a wait that times out
+// sets bit 0 of *err and the block stops.  With DIAG the block writes one row
+// of ZR_VORT_SUMS vorticity sums over its points to diag[blockIdx.x], for the
+// statistics of the state the step starts from.
+//   What bounds it (ncu, 512-point lines): issue 58%, shared-memory wavefronts
+// 59%.  Against a block of NPH warps of which NOUT run the forward transforms
+// after a products phase (two more barriers, NPH - NOUT warps idle): 512^3 one
+// scalar 2.52 -> 2.08 ms, 256^3 one scalar 0.380 -> 0.314, two scalars 0.725 ->
+// 0.402 ms (there one block per SM before).  In FP64 the forward warps' reads
+// of the factors (96 lines of 512 bytes per product) bound phase A: 512^3 two
+// scalars 5.95 ms against 5.10 of k_zws.
 template <typename T, int N, int NPH, int NRAW, bool DIAG = false, bool MB = false>
-__global__ void __launch_bounds__(NPH * 32, (sizeof(T) == 4 && NPH <= 9) ? (N <= 192 ? 4 : 3) : (N <= 192 ? 2 : 1))
-k_zreg(const __grid_constant__ FieldSet<T> f, const __grid_constant__ ZRecipeSet zr, int nout, long long npairs,
-       int ncp, int nkz, T scale, T alpha, double dkz, const V2<T> *__restrict__ tw, unsigned *__restrict__ err,
-       double *__restrict__ diag, long long mpairs, long long ms) {
+__global__ void __launch_bounds__(ZPipe<T, N, NPH>::NT, ZPipe<T, N, NPH>::MINB)
+k_zpipe(const __grid_constant__ FieldSet<T> f, const __grid_constant__ ZRecipeSet zr, long long npairs, int ncp,
+        int nkz, T scale, T alpha, double dkz, const V2<T> *__restrict__ tw, unsigned *__restrict__ err,
+        double *__restrict__ diag, long long mpairs, long long ms) {
     using V = V2<T>;
     using Z = ZRCfg<T, N>;
-    constexpr int E = Z::E, SCR = Z::SCR;
+    using C = ZPipe<T, N, NPH>;
+    constexpr int E = Z::E, ST = zl_stride<T, N>();
     double acc[DIAG ? ZR_VORT_SUMS : 1] = {};
     const int rawf = 2 * ncp;
     const unsigned raw_bytes = (unsigned)(rawf * sizeof(V));
     extern __shared__ __align__(16) unsigned char smem_raw[];
     V *tws = reinterpret_cast<V *>(smem_raw);
-    V *scr_all = tws + Z::LOGE * 32;
-    V *raw = scr_all + NPH * SCR;
+    V *lines = tws + Z::LOGE * 32;
+    V *fscr = lines + NPH * C::LINE;
+    V *raw = fscr + C::NOUT * C::FSCR;
     uint64_t *bar = reinterpret_cast<uint64_t *>(raw + NRAW * rawf);
     T *tkz = reinterpret_cast<T *>(bar + 2);   // kz wavenumbers of the kept modes (ncp entries)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    long long pair = blockIdx.x;
-    if (pair >= npairs) return;   // uniform for the block
-    for (int i = threadIdx.x; i < Z::LOGE * 32; i += blockDim.x) tws[i] = tw[Z::tw_index(i)];
-    for (int k = threadIdx.x; k < ncp; k += blockDim.x) tkz[k] = (T)wavenum(k, N, dkz);
-    unsigned keep = 0;   // bit m: mode min(n, N - n) of element n = lane + 32 m is kept
-#pragma unroll
-    for (int m = 0; m < E; ++m) {
-        const int n = (threadIdx.x & 31) + 32 * m;
-        keep |= ((2 * n <= N ? n : N - n) < nkz ? 1u : 0u) << m;
-    }
+    long long next = blockIdx.x;
+    if (next >= npairs) return;   // uniform for the block
+    for (int i = threadIdx.x; i < Z::LOGE * 32; i += C::NT) tws[i] = tw[Z::tw_index(i)];
+    for (int k = threadIdx.x; k < ncp; k += C::NT) tkz[k] = (T)wavenum(k, N, dkz);
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
         mbar_fence_init();
@@ -562,109 +658,171 @@ k_zreg(const __grid_constant__ FieldSet<T> f, const __grid_constant__ ZRecipeSet
     auto issue = [&](long long p, bool withhold = false) {
         mbar_arrive_expect_tx(bar, NRAW * raw_bytes);
         if (!withhold)
-            for (int q = 0; q < NRAW; ++q) bulk_g2s(raw + q * rawf, f.p[q] + pair_offset<MB>(p, mpairs, ms, rawf), raw_bytes, bar);
+            for (int q = 0; q < NRAW; ++q)
+                bulk_g2s(raw + q * rawf, f.p[q] + pair_offset<MB>(p, mpairs, ms, rawf), raw_bytes, bar);
     };
-    if (threadIdx.x == 0) issue(pair, wc.withhold);
-    unsigned parity = 0;
-    const ZRecipe rc = zr.q[warp];
-    const int kind = zr_kind(rc);
-    V *scr = scr_all + warp * SCR;   // transposes, then this warp's physical quantity
-    for (; pair < npairs; pair += gridDim.x) {
-        const bool ok = mbar_wait_bounded(bar, parity, wc.limit);
-        if (__syncthreads_or(!ok)) {
-            if (threadIdx.x == 0) atomicOr(err, 1u);
-            mbar_wait_bounded(bar, parity, wc.limit);   // let an overdue copy land before leaving
-            return;
-        }
-        parity ^= 1u;
-        V x[E];
-        if constexpr (sizeof(T) == 8 && E % 2 == 0)   // measured: faster in FP64; in FP32 the general form keeps 72 registers
-            zr_pack_any<T, N>(kind, lane, x, rc, raw, rawf, ncp, nkz, keep, tkz);
-        else
-            zr_pack<T, N>(lane, x, rc, raw + rc.r[0] * rawf, rc.r[1] >= 0 ? raw + rc.r[1] * rawf : nullptr, ncp, keep,
-                          tkz);
-        __syncthreads();   // staging consumed; the previous pair's products are read
-        if (threadIdx.x == 0 && pair + gridDim.x < npairs) {
-            fence_proxy_async_smem();
-            issue(pair + gridDim.x);
-        }
-        zr_fft<T, N, +1>(lane, x, scr, tws);   // ends its scratch reads with __syncwarp
+    if (threadIdx.x == 0) issue(next, wc.withhold);
+    const int step = gridDim.x;
+    // barriers 1 (A ends) and 2 (B ends) over the whole block, reached from both loops the same number of times
+    const SyncNamed end_b{2, C::NT};
+    if (warp < NPH) {   // inverse warps: pair `next`
+        const ZRecipe rc = zr.q[warp];
+        const T ls = zr_line_scale<T, NPH>(warp, scale);
+        const V lsc = V{ls, ls};
+        V *const line = lines + warp * C::LINE;
+        unsigned parity = 0;
+        for (; next < npairs; next += step) {
+            V x[E];
+            const bool ok = mbar_wait_bounded(bar, parity, wc.limit);
+            zl_pack<T, N>(lane, x, rc, raw + rc.r[0] * rawf, raw + rc.r[1] * rawf, ncp, nkz, tkz);
+            if (bar_named_or(1, C::NT, !ok)) {   // the raw lines and the physical lines have been read
+                if (threadIdx.x == 0) {
+                    atomicOr(err, 1u);
+                    mbar_wait_bounded(bar, parity, wc.limit);   // let an overdue copy land before leaving
+                }
+                return;
+            }
+            parity ^= 1u;
+            if (threadIdx.x == 0 && next + step < npairs) {
+                fence_proxy_async_smem();
+                issue(next + step);
+            }
+            zr_fft<T, N, +1>(lane, x, line, tws);   // ends its scratch reads with __syncwarp
+            V *d = line + zl_base<T, N>(lane);
 #pragma unroll
-        for (int q = 0; q < E; ++q) scr[Z::pidx(zr_out_index<T, N>(lane, q))] = cscale(x[q], scale);
-        __syncthreads();   // every physical quantity on chip
-        zr_products<T, N, NPH, DIAG>(scr_all, scr_all, alpha, acc);
-        __syncthreads();   // products in the scratch lines of warps 0 .. nout-1
-        if (warp < nout) {   // z R2C of product `warp`, written over raw field `warp` of the pair
-#pragma unroll
-            for (int m = 0; m < E; ++m) x[m] = scr[Z::pidx(lane + 32 * m)];
-            __syncwarp();
-            zr_fft<T, N, -1>(lane, x, scr, tws);
-            zr_store_r2c<T, N>(lane, x, scr, f.p[warp] + pair_offset<MB>(pair, mpairs, ms, rawf), ncp);
+            for (int q = 0; q < E; ++q) d[q * ST] = lmul(x[q], lsc);
+            end_b();   // the physical lines of `next` are complete
+        }
+        bar_named_or(1, C::NT, false);   // the forward warps' last pair
+    } else {            // forward warps: the pair before
+        const int q = warp - NPH;
+        V *const scr = fscr + q * C::FSCR;
+        if (bar_named_or(1, C::NT, false)) return;
+        end_b();
+        for (;;) {
+            V x[E];
+            zl_product<T, N, NPH, DIAG>(q, lane, x, lines, alpha, scale, acc);
+            if (bar_named_or(1, C::NT, false)) return;
+            zr_fft_rev<T, N, -1>(lane, x, scr, tws);
+            zl_unpack<T, N>(lane, x, f.p[q] + pair_offset<MB>(next, mpairs, ms, rawf), ncp);
+            next += step;
+            if (next >= npairs) break;
+            end_b();
         }
     }
-    if constexpr (DIAG) {   // warp shuffles, then the block's warps in order
-        __shared__ double red[ZR_VORT_SUMS][NPH];
+    if constexpr (DIAG) {   // the sums lie in the lanes of one warp: added in a fixed order
+        if (warp == NPH) {
 #pragma unroll
-        for (int q = 0; q < ZR_VORT_SUMS; ++q) {
-            double v = acc[q];
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if (lane == 0) red[q][warp] = v;
-        }
-        __syncthreads();
-        if (threadIdx.x < ZR_VORT_SUMS) {
-            double v = 0.0;
-            for (int w = 0; w < NPH; ++w) v += red[threadIdx.x][w];
-            diag[blockIdx.x * ZR_VORT_SUMS + threadIdx.x] = v;
+            for (int q = 0; q < ZR_VORT_SUMS; ++q) {
+                double v = acc[q];
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+                if (lane == 0) diag[blockIdx.x * ZR_VORT_SUMS + q] = v;
+            }
         }
     }
 }
 
-// Warp-specialised form of k_zreg (same arguments, same results): NPH inverse
-// warps and nout forward warps per block, each with its own scratch line.
-// Per line pair p, between two block barriers, the inverse warps unpack and
-// transform the quantities of p (each leaving its physical quantity in its
-// own line) while the forward warps transform and store the products of the
-// block's previous pair (held in their own lines); after the first barrier
-// the whole block forms the products of p into the forward warps' lines.
-// Every warp thus runs one length-N transform per pair instead of nout of
-// NPH warps running the forward ones alone.  The raw lines of the next pair
-// are requested as soon as every inverse warp has unpacked (named barrier 1);
-// a wait that times out sets bit 0 of *err and the block stops.  FP32 with 9
-// quantities: 13 warps, 72 registers, two blocks per SM; FP64 with 9 or 12
-// quantities: 13 or 17 warps, one block per SM (k_zreg: 9 or 12).
-template <int NPH> __host__ __device__ constexpr int zws_nout() { return NPH >= 12 ? 5 : 4; }
-template <typename T, int N, int NPH, int NRAW, bool MB = false>
-__global__ void __launch_bounds__((NPH + zws_nout<NPH>()) * 32, sizeof(T) == 4 ? 2 : 1)
-k_zws(const __grid_constant__ FieldSet<T> f, const __grid_constant__ ZRecipeSet zr, int nout, long long npairs,
-      int ncp, int nkz, T scale, T alpha, double dkz, const V2<T> *__restrict__ tw, unsigned *__restrict__ err,
-      long long mpairs, long long ms) {
-    constexpr int NOUT = zws_nout<NPH>();   // products (the host checks nout)
-    static_assert(NPH == 9 || NPH == 12, "k_zws serves 9 or 12 physical quantities");
+// Products of one line pair by the whole block (k_zws): quantities in the
+// lines `phys`, product f into line f of `out` (both stride SCR).  A thread
+// takes both lines' values of a point, or one of them where that fills the
+// rounds better (N = 512 with 13 warps: 3 rounds of single values against 2
+// of double the work).  DIAG adds the vorticity sums to acc.
+template <typename T, int N, int NPH, int NT, bool DIAG>
+__device__ __forceinline__ void zr_products(const V2<T> *phys, V2<T> *out, T alpha, T scale, double *acc) {
+    using Z = ZRCfg<T, N>;
+    constexpr bool HALF = (2 * N + NT - 1) / NT < 2 * ((N + NT - 1) / NT);
+    using W = std::conditional_t<HALF, T, V2<T>>;
+    constexpr int L = (HALF ? 2 : 1) * Z::SCR;
+    for (int i = threadIdx.x; i < (HALF ? 2 : 1) * N; i += NT) {
+        const int at = HALF ? 2 * Z::pidx(i >> 1) + (i & 1) : Z::pidx(i);
+        const W *p = reinterpret_cast<const W *>(phys) + at;
+        const W u = p[0], v = p[L], w = p[2 * L], o1 = p[3 * L], o2 = p[4 * L], o3 = p[5 * L];
+        const W sx = p[6 * L], sy = p[7 * L], sz = p[8 * L];
+        if constexpr (DIAG) {
+            const double s = zr_fold_scale<NPH>() ? (double)scale : 1.0;
+            auto add = [&](double ax, double ay, double az) {
+                acc[0] += sqrt(ax * ax + ay * ay + az * az);
+                acc[1] += ax * ax;
+                acc[2] += ay * ay;
+                acc[3] += az * az;
+            };
+            if constexpr (HALF) {
+                add(s * o1, s * o2, s * o3);
+            } else {
+                add(s * o1.x, s * o2.x, s * o3.x);
+                add(s * o1.y, s * o2.y, s * o3.y);
+            }
+        }
+        W *o = reinterpret_cast<W *>(out) + at;
+        o[0] = lfma(o2, w, lneg(lmul(o3, v)));
+        o[L] = lfma(o3, u, lneg(lmul(o1, w)));
+        o[2 * L] = lfma(o1, v, lneg(lmul(o2, u)));
+        o[3 * L] = lfma(w, sz, lfma(v, sy, lmul(u, sx)));
+        if constexpr (NPH >= 12) {
+            const W cx = p[9 * L], cy = p[10 * L], cz = p[11 * L];
+            W n = lfma(w, cz, lfma(v, cy, lmul(u, cx)));
+            if constexpr (NPH >= 14) {
+                const W dr = lfma(cz, sz, lfma(cy, sy, lfma(cx, sx, lmul(p[13 * L], p[12 * L]))));
+                W al;
+                if constexpr (HALF) al = alpha;
+                else al = W{alpha, alpha};
+                n = lfma(al, dr, n);
+            }
+            o[4 * L] = n;
+        }
+    }
+}
+
+// Block shape of k_zws: one line per warp, NPH inverse and NOUT forward ones.
+template <typename T, int N, int NPH> struct ZWs {
+    using Z = ZRCfg<T, N>;
+    static constexpr int NOUT = z_nout<NPH>(), NT = (NPH + NOUT) * 32;
+    // blocks per SM the registers are sized for
+    static constexpr int MINB = N == 512 ? 1 : N == 256 ? (NPH == 9 ? 2 : 1) : (NPH <= 12 ? 2 : 1);
+    __host__ __device__ static constexpr int smem_bytes(int nraw, int ncp) {
+        return (Z::LOGE * 32 + (NPH + NOUT) * Z::SCR + nraw * 2 * ncp) * (int)sizeof(V2<T>) + 16 + ncp * (int)sizeof(T);
+    }
+};
+
+// The fused z stage in FP64, same arguments and contract as k_zpipe (STAGED =
+// false: the staging does not fit, the inverse warps read the raw lines from
+// global memory).  Per line pair, between two block barriers, the inverse warps pack and transform the
+// quantities of pair p while the forward warps transform and store the
+// products of the pair before (held in their own lines); then the whole block
+// forms the products of p into the forward warps' lines.  The raw lines of the
+// next pair are requested as soon as every inverse warp has packed (named
+// barrier 1).
+//   What bounds it (ncu, 512-point lines): shared-memory wavefronts 59%, the
+// FP64 pipe 42%, with one block of 13 or 17 warps per SM.  Reading each raw
+// mode once (the mirrored half by shuffle), transforming the products in the
+// reversed flow graph and storing them from registers took 512^3 from 5.53 to
+// 5.10 ms (two scalars) and 4.59 to 4.24 ms (one), 192^3 from 0.375 to 0.330.
+template <typename T, int N, int NPH, int NRAW, bool DIAG = false, bool MB = false, bool STAGED = true>
+__global__ void __launch_bounds__(ZWs<T, N, NPH>::NT, ZWs<T, N, NPH>::MINB)
+k_zws(const __grid_constant__ FieldSet<T> f, const __grid_constant__ ZRecipeSet zr, long long npairs, int ncp, int nkz,
+      T scale, T alpha, double dkz, const V2<T> *__restrict__ tw, unsigned *__restrict__ err,
+      double *__restrict__ diag, long long mpairs, long long ms) {
     using V = V2<T>;
     using Z = ZRCfg<T, N>;
-    constexpr int E = Z::E, SCR = Z::SCR;
+    using C = ZWs<T, N, NPH>;
+    constexpr int E = Z::E, SCR = Z::SCR, ST = zl_stride<T, N>();
     constexpr unsigned NINV = NPH * 32;   // threads of the inverse warps (named barrier 1)
-    (void)nout;
+    constexpr bool FIXED = N == 512 && NPH >= 12;
+    double acc[DIAG ? ZR_VORT_SUMS : 1] = {};
     const int rawf = 2 * ncp;
     const unsigned raw_bytes = (unsigned)(rawf * sizeof(V));
     extern __shared__ __align__(16) unsigned char smem_raw[];
     V *tws = reinterpret_cast<V *>(smem_raw);
-    V *lines = tws + Z::LOGE * 32;           // NPH + NOUT scratch lines, one per warp
-    V *raw = lines + (NPH + NOUT) * SCR;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(raw + NRAW * rawf);
+    V *lines = tws + Z::LOGE * 32;   // NPH + NOUT lines, one per warp
+    V *raw = lines + (NPH + C::NOUT) * SCR;
+    uint64_t *bar = reinterpret_cast<uint64_t *>(raw + (STAGED ? NRAW * rawf : 0));
     T *tkz = reinterpret_cast<T *>(bar + 2);   // kz wavenumbers of the kept modes (ncp entries)
     __shared__ int stop;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     long long pair = blockIdx.x;
     if (pair >= npairs) return;   // uniform for the block
-    for (int i = threadIdx.x; i < Z::LOGE * 32; i += blockDim.x) tws[i] = tw[Z::tw_index(i)];
-    for (int k = threadIdx.x; k < ncp; k += blockDim.x) tkz[k] = (T)wavenum(k, N, dkz);
-    unsigned keep = 0;   // bit m: mode min(n, N - n) of element n = lane + 32 m is kept
-#pragma unroll
-    for (int m = 0; m < E; ++m) {
-        const int n = lane + 32 * m;
-        keep |= ((2 * n <= N ? n : N - n) < nkz ? 1u : 0u) << m;
-    }
+    for (int i = threadIdx.x; i < Z::LOGE * 32; i += C::NT) tws[i] = tw[Z::tw_index(i)];
+    for (int k = threadIdx.x; k < ncp; k += C::NT) tkz[k] = (T)wavenum(k, N, dkz);
     if (threadIdx.x == 0) {
         stop = 0;
         mbar_init(bar, 1);
@@ -676,59 +834,81 @@ k_zws(const __grid_constant__ FieldSet<T> f, const __grid_constant__ ZRecipeSet 
     auto issue = [&](long long p, bool withhold = false) {
         mbar_arrive_expect_tx(bar, NRAW * raw_bytes);
         if (!withhold)
-            for (int q = 0; q < NRAW; ++q) bulk_g2s(raw + q * rawf, f.p[q] + pair_offset<MB>(p, mpairs, ms, rawf), raw_bytes, bar);
+            for (int q = 0; q < NRAW; ++q)
+                bulk_g2s(raw + q * rawf, f.p[q] + pair_offset<MB>(p, mpairs, ms, rawf), raw_bytes, bar);
     };
-    if (threadIdx.x == 0) issue(pair, wc.withhold);
+    if (STAGED && threadIdx.x == 0) issue(pair, wc.withhold);
     unsigned parity = 0;
     const bool inv = warp < NPH;
     const ZRecipe rc = zr.q[inv ? warp : 0];
-    const int kind = zr_kind(rc);
     V *scr = lines + warp * SCR;
+    const T ls = zr_line_scale<T, NPH>(warp, scale);
+    const V lsc = V{ls, ls};
     long long prev = -1;
     for (;;) {
         if (inv) {
             if (pair < npairs) {
-                const bool ok = mbar_wait_bounded(bar, parity, wc.limit);
                 V x[E];
-                if constexpr (sizeof(T) == 8 && E % 2 == 0)   // as k_zreg
-                    zr_pack_any<T, N>(kind, lane, x, rc, raw, rawf, ncp, nkz, keep, tkz);
-                else
-                    zr_pack<T, N>(lane, x, rc, raw + rc.r[0] * rawf, rc.r[1] >= 0 ? raw + rc.r[1] * rawf : nullptr,
-                                  ncp, keep, tkz);
-                if (bar_named_or(1, NINV, !ok)) {   // every inverse warp has unpacked, or one gave up
+                bool ok = true;
+                if constexpr (STAGED) {
+                    ok = mbar_wait_bounded(bar, parity, wc.limit);
+                    zl_pack<T, N, FIXED>(lane, x, rc, raw + rc.r[0] * rawf, raw + rc.r[1] * rawf, ncp, nkz, tkz);
+                } else {
+                    const long long off = pair_offset<MB>(pair, mpairs, ms, rawf);
+                    zl_pack<T, N>(lane, x, rc, f.p[rc.r[0]] + off, f.p[rc.r[1] >= 0 ? rc.r[1] : 0] + off, ncp, nkz, tkz);
+                }
+                if (STAGED && bar_named_or(1, NINV, !ok)) {   // every inverse warp has packed, or one gave up
                     if (threadIdx.x == 0) {
                         stop = 1;
                         mbar_wait_bounded(bar, parity, wc.limit);   // let an overdue copy land before leaving
                     }
                 } else {
                     parity ^= 1u;
-                    if (threadIdx.x == 0 && pair + gridDim.x < npairs) {
+                    if (STAGED && threadIdx.x == 0 && pair + gridDim.x < npairs) {
                         fence_proxy_async_smem();
                         issue(pair + gridDim.x);
                     }
                     zr_fft<T, N, +1>(lane, x, scr, tws);   // ends its scratch reads with __syncwarp
+                    V *d = scr + zl_base<T, N>(lane);
 #pragma unroll
-                    for (int q = 0; q < E; ++q) scr[Z::pidx(zr_out_index<T, N>(lane, q))] = cscale(x[q], scale);
+                    for (int q = 0; q < E; ++q) d[q * ST] = lmul(x[q], lsc);
                 }
             }
         } else if (prev >= 0) {   // z R2C of product warp - NPH of the previous pair
             V x[E];
+            const V *d = scr + zl_base<T, N>(lane);
 #pragma unroll
-            for (int m = 0; m < E; ++m) x[m] = scr[Z::pidx(lane + 32 * m)];
+            for (int q = 0; q < E; ++q) x[q] = d[q * ST];
             __syncwarp();
-            zr_fft<T, N, -1>(lane, x, scr, tws);
-            zr_store_r2c<T, N>(lane, x, scr, f.p[warp - NPH] + pair_offset<MB>(prev, mpairs, ms, rawf), ncp);
+            zr_fft_rev<T, N, -1>(lane, x, scr, tws);
+            zl_unpack<T, N>(lane, x, f.p[warp - NPH] + pair_offset<MB>(prev, mpairs, ms, rawf), ncp);
         }
         __syncthreads();   // quantities of `pair` in the inverse warps' lines; the forward lines are free
-        if (stop) {
+        if (STAGED && stop) {
             if (threadIdx.x == 0) atomicOr(err, 1u);
             return;
         }
         if (pair >= npairs) break;
-        zr_products<T, N, NPH>(lines, lines + NPH * SCR, alpha);
+        zr_products<T, N, NPH, C::NT, DIAG>(lines, lines + NPH * SCR, alpha, scale, acc);
         __syncthreads();   // products of `pair` in the forward warps' lines
         prev = pair;
         pair += gridDim.x;
+    }
+    if constexpr (DIAG) {   // warp shuffles, then the block's warps in order
+        constexpr int NW = NPH + C::NOUT;
+        __shared__ double red[ZR_VORT_SUMS][NW];
+#pragma unroll
+        for (int q = 0; q < ZR_VORT_SUMS; ++q) {
+            double v = acc[q];
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) red[q][warp] = v;
+        }
+        __syncthreads();
+        if (threadIdx.x < ZR_VORT_SUMS) {
+            double v = 0.0;
+            for (int w = 0; w < NW; ++w) v += red[threadIdx.x][w];
+            diag[blockIdx.x * ZR_VORT_SUMS + threadIdx.x] = v;
+        }
     }
 }
 
