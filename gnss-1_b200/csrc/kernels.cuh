@@ -335,7 +335,7 @@ __device__ __forceinline__ void unpack_r2c(int lane, const V2<T> *line, V2<T> *_
 
 template <typename T, int N, int DIR>
 __global__ void __launch_bounds__(ZWARPS * 32, 2)
-k_zpass(FieldSet<T> f, long long nlines, int nz2, T scale, const V2<T> *__restrict__ tw) {
+k_zpass(const __grid_constant__ FieldSet<T> f, long long nlines, int nz2, T scale, const V2<T> *__restrict__ tw) {
     using V = V2<T>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

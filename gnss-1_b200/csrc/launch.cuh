@@ -1,5 +1,6 @@
 // launch.cuh -- helpers shared by the launchers.
 #pragma once
+#include <algorithm>
 #include <atomic>
 #include <type_traits>
 

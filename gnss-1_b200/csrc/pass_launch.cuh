@@ -4,6 +4,7 @@
 #include "launch.cuh"
 #include "passd.cuh"
 #include "passtc.cuh"
+#include "zreg.cuh"
 
 template <typename T> static const V2<T> *pass_twiddles(const PassPtrs<T> &, const void *tw) {
     return reinterpret_cast<const V2<T> *>(tw);
@@ -106,15 +107,28 @@ template <typename T, int N> struct PassLaunch {
     }
     static cudaError_t zpass(int dir, const FieldSet<T> &f, int nfields, long long nlines, int nz2, T scale,
                              const void *tw, cudaStream_t s) {
-        using C = ZCfg<T, N>;
-        long long npairs = (nlines + 1) / 2;
-        dim3 grid((unsigned)((npairs + ZWARPS - 1) / ZWARPS), (unsigned)nfields);
-        const V2<T> *t = reinterpret_cast<const V2<T> *>(tw);
-        auto kern = dir < 0 ? k_zpass<T, N, -1> : k_zpass<T, N, +1>;
-        cudaError_t e = prep_smem(kern, C::SMEM);
-        if (e != cudaSuccess) return e;
-        kern<<<grid, ZWARPS * 32, C::SMEM, s>>>(f, nlines, nz2, scale, t);
-        return cudaGetLastError();
+        if constexpr (zr_size(N)) {
+            using Z = ZRCfg<T, N>;
+            const int smem = (Z::LOGE * 32 + ZLINE_WARPS * Z::SCR) * (int)sizeof(V2<T>);
+            auto kern = dir < 0 ? k_zline<T, N, -1> : k_zline<T, N, +1>;
+            cudaError_t e = prep_smem(kern, smem);
+            if (e != cudaSuccess) return e;
+            const long long np = nlines / 2;
+            const long long blocks = (np + ZLINE_WARPS - 1) / ZLINE_WARPS;
+            kern<<<dim3((unsigned)std::min<long long>(blocks, 148LL * 16), (unsigned)nfields), ZLINE_WARPS * 32, smem, s>>>(
+                f, (int)np, nz2, scale, reinterpret_cast<const V2<T> *>(tw));
+            return cudaGetLastError();
+        } else {
+            using C = ZCfg<T, N>;
+            long long npairs = (nlines + 1) / 2;
+            dim3 grid((unsigned)((npairs + ZWARPS - 1) / ZWARPS), (unsigned)nfields);
+            const V2<T> *t = reinterpret_cast<const V2<T> *>(tw);
+            auto kern = dir < 0 ? k_zpass<T, N, -1> : k_zpass<T, N, +1>;
+            cudaError_t e = prep_smem(kern, C::SMEM);
+            if (e != cudaSuccess) return e;
+            kern<<<grid, ZWARPS * 32, C::SMEM, s>>>(f, nlines, nz2, scale, t);
+            return cudaGetLastError();
+        }
     }
 };
 

@@ -523,6 +523,65 @@ template <typename T, int N> __device__ __forceinline__ int zl_base(int lane) {
 template <typename T, int N> __host__ __device__ constexpr int zl_stride() {
     return ZRCfg<T, N>::SHFL ? 1 : ZRCfg<T, N>::E;
 }
+// The plain z pass (gnss_forward / gnss_inverse) with register transforms, one
+// warp per pair of lines of one field: DIR < 0 real padded lines -> nz2 complex
+// per line, DIR > 0 the reverse, scaled, with the padding reals zeroed; in
+// place.  Modes go between global memory and registers, points through a
+// shared line, so that both sides are coalesced.  A field has an even number
+// of lines.
+//   Measured against k_zpass (a shared-memory round trip per radix-8 stage):
+// see the launcher.
+constexpr int ZLINE_WARPS = 4;
+template <typename T, int N, int DIR>
+__global__ void __launch_bounds__(ZLINE_WARPS * 32)
+k_zline(const __grid_constant__ FieldSet<T> f, int npairs, int nz2, T scale, const V2<T> *__restrict__ tw) {
+    using V = V2<T>;
+    using Z = ZRCfg<T, N>;
+    constexpr int E = Z::E, ST = zl_stride<T, N>(), M = N / 32;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    V *tws = reinterpret_cast<V *>(smem_raw);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    V *line = tws + Z::LOGE * 32 + warp * Z::SCR;
+    for (int i = threadIdx.x; i < Z::LOGE * 32; i += ZLINE_WARPS * 32) tws[i] = tw[Z::tw_index(i)];
+    __syncthreads();
+    V *field = f.p[blockIdx.y];
+    for (int pair = blockIdx.x * ZLINE_WARPS + warp; pair < npairs; pair += gridDim.x * ZLINE_WARPS) {
+        V *modes = field + (long long)pair * 2 * nz2;
+        T *ra = reinterpret_cast<T *>(modes), *rb = ra + 2 * nz2;
+        V *at = line + zl_base<T, N>(lane);
+        V x[E];
+        if constexpr (DIR < 0) {
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                const int n = lane + 32 * m;
+                line[Z::pidx(n)] = V{ra[n], rb[n]};
+            }
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < E; ++q) x[q] = at[q * ST];
+            __syncwarp();
+            zr_fft_rev<T, N, -1>(lane, x, line, tws);
+            zl_unpack<T, N>(lane, x, modes, nz2);
+        } else {
+            const ZRecipe rc{{0, -1}, {0, 0}, {1, 1}, {0, 0}};
+            zl_pack_form<T, N, 0>(lane, x, rc, modes, modes, nz2, nz2, nullptr);
+            zr_fft<T, N, +1>(lane, x, line, tws);
+#pragma unroll
+            for (int q = 0; q < E; ++q) at[q * ST] = x[q];
+            __syncwarp();
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                const int n = lane + 32 * m;
+                const V z = line[Z::pidx(n)];
+                ra[n] = z.x * scale;
+                rb[n] = z.y * scale;
+            }
+            if (lane < 2 * nz2 - N) ra[N + lane] = rb[N + lane] = T(0);
+        }
+        __syncwarp();   // the line is free
+    }
+}
+
 // The inverse transforms leave the lines unscaled; their 1/N^3 enters as
 // scale^2 on u, v, w (one factor of every product), except with the colloid
 // term, whose products have none of them: there every line is scaled.
