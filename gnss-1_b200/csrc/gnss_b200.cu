@@ -479,31 +479,36 @@ static gnss_status nonlinear_and_update(gnss_ctx *c, const gnss_fields *state, v
     }
     {
         StageTimer t(c, s, 5);
-        // one warp per kept (ky, kx) row; 8 blocks of 8 warps per SM
+        // one warp per kept (ky, kx) row, or half a warp where rows are short (the sphere leaves 2/3 of nkz modes on
+        // average, and the last 32 lanes of a row are half empty); 8 blocks of 8 warps per SM
+        const int lpr = c->nkz > 96 ? 32 : 16;
         const long long nrows = (long long)c->ky_keep.count() * c->kx_keep.count() * bt.nmem;
         const int full_rows = (uc.scheme == GNSS_SCHEME_CNAB2 && uc.euler) ? 1 : 0;
-        long long nblk = std::min<long long>((nrows + 7) / 8, 8LL * c->nsm);
+        const long long nwarps = (nrows * lpr + 31) / 32;
+        long long nblk = std::min<long long>((nwarps + 7) / 8, 8LL * c->nsm);
+        const bool cn = uc.scheme == GNSS_SCHEME_CNAB2, one = sizeof(T) == 4 && uc.nf == 4;
         if (bt.nmem > 1) {   // a batch (no statistics): per-member coefficients and mean lines
-            auto kb = uc.scheme == GNSS_SCHEME_CNAB2 ? k_update_batch<T, GNSS_SCHEME_CNAB2>
-                                                     : k_update_batch<T, GNSS_SCHEME_RK3IF>;
+            auto kb = cn ? (one ? k_update_batch<T, GNSS_SCHEME_CNAB2, 4> : k_update_batch<T, GNSS_SCHEME_CNAB2, 5>)
+                         : (one ? k_update_batch<T, GNSS_SCHEME_RK3IF, 4> : k_update_batch<T, GNSS_SCHEME_RK3IF, 5>);
             CK(c, launch_dep(kb, dim3((unsigned)nblk), dim3(256), 0, s, SF, H, R, g, c->kx_keep, c->ky_keep, c->nkz,
-                             c->ncp, uc, full_rows, *bt.mc, bt.nmem, bt.ms_sh, bt.ms_scr));
+                             c->ncp, uc, full_rows, *bt.mc, bt.nmem, bt.ms_sh, bt.ms_scr, lpr));
             return GNSS_OK;
         }
         if (stats_dst) {   // statistics of the new state summed by the update itself (one partial row per block)
             nblk = std::min<long long>(nblk, STAT_BLOCKS);
-            auto ku = uc.scheme == GNSS_SCHEME_CNAB2 ? k_update<T, GNSS_SCHEME_CNAB2, true>
-                                                     : k_update<T, GNSS_SCHEME_RK3IF, true>;
+            auto ku = cn ? (one ? k_update<T, GNSS_SCHEME_CNAB2, 4, true> : k_update<T, GNSS_SCHEME_CNAB2, 5, true>)
+                         : (one ? k_update<T, GNSS_SCHEME_RK3IF, 4, true> : k_update<T, GNSS_SCHEME_RK3IF, 5, true>);
             CK(c, launch_dep(ku, dim3((unsigned)nblk), dim3(256), 0, s, SF, H, R, g, c->kx_keep, c->ky_keep, c->nkz,
-                             c->ncp, uc, full_rows, c->stat_part, c->mean64));
+                             c->ncp, uc, full_rows, c->stat_part, c->mean64, lpr));
             c->launches++;
             CK(c, launch_dep(k_stats_final, dim3(1), dim3(STAT_SUMS * 32), 0, s, (const double *)c->stat_part,
                              (int)nblk, stats_dst));
             return GNSS_OK;
         }
-        auto ku = uc.scheme == GNSS_SCHEME_CNAB2 ? k_update<T, GNSS_SCHEME_CNAB2> : k_update<T, GNSS_SCHEME_RK3IF>;
+        auto ku = cn ? (one ? k_update<T, GNSS_SCHEME_CNAB2, 4> : k_update<T, GNSS_SCHEME_CNAB2, 5>)
+                     : (one ? k_update<T, GNSS_SCHEME_RK3IF, 4> : k_update<T, GNSS_SCHEME_RK3IF, 5>);
         CK(c, launch_dep(ku, dim3((unsigned)nblk), dim3(256), 0, s, SF, H, R, g, c->kx_keep, c->ky_keep, c->nkz,
-                         c->ncp, uc, full_rows, (double *)nullptr, c->mean64));
+                         c->ncp, uc, full_rows, (double *)nullptr, c->mean64, lpr));
     }
     return GNSS_OK;
 }

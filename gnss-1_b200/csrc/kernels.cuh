@@ -638,7 +638,7 @@ struct MemberCoef {
     double2 *mean[MAXM];    // FP32 contexts: the member's FP64 mean-profile line (or null)
 };
 
-// One warp per (ky, kx) row of the kept box, lanes along kz.  The arithmetic
+// One warp (nkz > 96) or half a warp per (ky, kx) row of the kept box, lanes along kz.  The arithmetic
 // follows makeRHS / deAlias / timestep / update (solver.cu:461-657) with the
 // divisions by k^2 and by (1 + dt k^2/(2 num)) done once as reciprocals.
 // Rows are enumerated in the kept box (kept ky, kept kx); nl is the compact
@@ -668,12 +668,12 @@ struct MemberCoef {
 // of STAT_SUMS partials per block to `partial`; for a state that is zero
 // outside the dealiasing sphere (the precondition of the step) they equal the
 // sums over the whole field.
-template <typename T, int SCHEME, bool STATS, bool BATCH>
+template <typename T, int SCHEME, int NF, bool STATS, bool BATCH>
 __device__ __forceinline__ void k_update_body(const FieldSet<T> &state, const FieldSet<T> &hist, const FieldSet<T> &nl,
                                               const Geom &g, KeepMap kx_keep, KeepMap ky_keep, int nkz, int ncp,
                                               const UpdCoef &c, int full_rows, double *__restrict__ partial,
                                               double2 *__restrict__ mean0, const MemberCoef *mc, int nmem,
-                                              long long ms_sh, long long ms_nl) {
+                                              long long ms_sh, long long ms_nl, int lpr) {
     using V = V2<T>;
     pdl_wait();
     pdl_trigger();
@@ -682,10 +682,16 @@ __device__ __forceinline__ void k_update_body(const FieldSet<T> &state, const Fi
     const int mrows = nky * nkx;   // rows of one member
     const int nrows = mrows * nmem;
     const int lane = threadIdx.x & 31;
-    const int nwarp = (int)((gridDim.x * blockDim.x) >> 5);
+    // lpr lanes per row (32, or 16: two rows per warp)
+    const int rpw = 32 / lpr, klane = lane & (lpr - 1);
+    const int step = (int)((gridDim.x * blockDim.x) >> 5) * rpw;
+    // FP64 takes the number of fields at run time (with it fixed the 512^3 update with two scalars measured 0.89
+    // against 0.75 ms: the loads of a mode no longer all go out first)
+    const int nf = sizeof(T) == 4 ? NF : c.nf;
     const bool read_hist = (SCHEME == 0) ? !c.euler : (c.substep > 0);
-    const int nf = c.nf;
-    for (int brow = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); brow < nrows; brow += nwarp) {
+    for (int wrow = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * rpw; wrow < nrows; wrow += step) {
+        const bool have = wrow + (lpr == 32 ? 0 : lane >> 4) < nrows;
+        const int brow = have ? wrow + (lpr == 32 ? 0 : lane >> 4) : wrow;
         const int mi = BATCH ? brow / mrows : 0;
         const int row = BATCH ? brow - mi * mrows : brow;
         const int kyc = row / nkx, kxc = row - kyc * nkx;
@@ -695,9 +701,9 @@ __device__ __forceinline__ void k_update_body(const FieldSet<T> &state, const Fi
         const long long jbase = (long long)row * ncp + (BATCH ? mi * ms_nl : 0);                    // nonlinear term
         double2 *const mean = BATCH ? mc->mean[mi] : mean0;
         const double c_dt = BATCH ? mc->dt[mi] : c.dt;
-        for (int k0 = 0; k0 < nkz; k0 += 32) {
-            const int kzi = k0 + lane;
-            const bool inrow = kzi < nkz;
+        for (int k0 = 0; k0 < nkz; k0 += lpr) {
+            const int kzi = k0 + klane;
+            const bool inrow = have && kzi < nkz;
             const double k3 = wavenum(kzi, g.nz, g.dkz);
             const double ksq = ksq3(k1, k2, k3);
             const bool masked = ksq > g.kmax2;
@@ -708,7 +714,7 @@ __device__ __forceinline__ void k_update_body(const FieldSet<T> &state, const Fi
                 // deAlias of the state and of the right-hand side (solver.cu:36, 756)
                 if (full_rows) {
 #pragma unroll
-                    for (int q = 0; q < 5; ++q) {
+                    for (int q = 0; q < NF; ++q) {
                         if (q < nf) {
                             state.p[q][idx] = V{T(0), T(0)};
                             hist.p[q][idx] = V{T(0), T(0)};
@@ -717,9 +723,9 @@ __device__ __forceinline__ void k_update_body(const FieldSet<T> &state, const Fi
                 }
                 continue;
             }
-            V a[5], f[5], h[5];
+            V a[NF], f[NF], h[NF];
 #pragma unroll
-            for (int q = 0; q < 5; ++q) {
+            for (int q = 0; q < NF; ++q) {
                 a[q] = V{T(0), T(0)};
                 f[q] = V{T(0), T(0)};
                 h[q] = V{T(0), T(0)};
@@ -731,10 +737,10 @@ __device__ __forceinline__ void k_update_body(const FieldSet<T> &state, const Fi
             }
             // makeRHS: (k k^T / k^2 - I) N for the velocity, -N for the scalars,
             // zero at k = 0 (solver.cu:461-521)
-            double R[5][2];
+            double R[NF][2];
             if (kxi == 0 && kyi == 0 && kzi == 0) {
 #pragma unroll
-                for (int q = 0; q < 5; ++q) R[q][0] = R[q][1] = 0.0;
+                for (int q = 0; q < NF; ++q) R[q][0] = R[q][1] = 0.0;
             } else {
                 const double ik = 1.0 / ksq;
                 const double pr = (k1 * (double)a[0].x + k2 * (double)a[1].x + k3 * (double)a[2].x) * ik;
@@ -746,7 +752,7 @@ __device__ __forceinline__ void k_update_body(const FieldSet<T> &state, const Fi
                 R[2][0] = k3 * pr - (double)a[2].x;
                 R[2][1] = k3 * pi - (double)a[2].y;
 #pragma unroll
-                for (int q = 3; q < 5; ++q) {
+                for (int q = 3; q < NF; ++q) {
                     R[q][0] = -(double)a[q].x;
                     R[q][1] = -(double)a[q].y;
                 }
@@ -754,10 +760,23 @@ __device__ __forceinline__ void k_update_body(const FieldSet<T> &state, const Fi
             V sv[STATS ? 5 : 1];   // the stored new state (the statistics read these values)
             // the mean-profile line in FP64 (FP32 contexts)
             const bool mline = sizeof(T) == 4 && mean != nullptr && kxi == 0 && kzi == 0;
+            // the viscous factors; u, v, w share one diffusivity (FP32 keeps them: FP64 has no registers to spare and
+            // is bound by its loads)
+            double am = 0.0, ib = 0.0, ex = 0.0;
+            if constexpr (STATS && NF < 5) sv[4] = V{T(0), T(0)};
 #pragma unroll
-            for (int q = 0; q < 5; ++q) {
+            for (int q = 0; q < NF; ++q) {
                 if constexpr (STATS) sv[q] = V{T(0), T(0)};
                 if (q >= nf) break;
+                if (sizeof(T) == 8 || q == 0 || q >= 3) {
+                    if constexpr (SCHEME == 0) {
+                        const double hk = (BATCH ? mc->hnum[mi][q] : c.hnum[q]) * ksq;
+                        am = 1.0 - hk;
+                        ib = 1.0 / (1.0 + hk);
+                    } else {
+                        ex = exp(-(BATCH ? mc->nu[mi][q] : c.nu[q]) * ksq * c.alph * c_dt);
+                    }
+                }
                 double fr = (double)f[q].x, fi = (double)f[q].y;
                 double hr = (double)h[q].x, hi = (double)h[q].y;
                 if (mline) {
@@ -771,9 +790,6 @@ __device__ __forceinline__ void k_update_body(const FieldSet<T> &state, const Fi
                 double nr, ni, gr, gi;   // new state and new history
                 if constexpr (SCHEME == 0) {
                     // eulerKernel_mgpu / adamsBashforthKernel_mgpu (solver.cu:547-585)
-                    const double hk = (BATCH ? mc->hnum[mi][q] : c.hnum[q]) * ksq;
-                    const double am = 1.0 - hk;
-                    const double ib = 1.0 / (1.0 + hk);
                     if (c.euler) {
                         nr = (am * fr + c_dt * R[q][0]) * ib;
                         ni = (am * fi + c_dt * R[q][1]) * ib;
@@ -784,11 +800,10 @@ __device__ __forceinline__ void k_update_body(const FieldSet<T> &state, const Fi
                     gr = R[q][0];   // updateKernel_mgpu (solver.cu:618-637)
                     gi = R[q][1];
                 } else {
-                    const double E = exp(-(BATCH ? mc->nu[mi][q] : c.nu[q]) * ksq * c.alph * c_dt);
-                    nr = E * (fr + c.gam * c_dt * R[q][0] + hr);
-                    ni = E * (fi + c.gam * c_dt * R[q][1] + hi);
-                    gr = c.zet_next * c_dt * E * R[q][0];
-                    gi = c.zet_next * c_dt * E * R[q][1];
+                    nr = ex * (fr + c.gam * c_dt * R[q][0] + hr);
+                    ni = ex * (fi + c.gam * c_dt * R[q][1] + hi);
+                    gr = c.zet_next * c_dt * ex * R[q][0];
+                    gi = c.zet_next * c_dt * ex * R[q][1];
                 }
                 state.p[q][idx] = V{(T)nr, (T)ni};
                 if constexpr (STATS) sv[q] = V{(T)nr, (T)ni};
@@ -833,22 +848,24 @@ __device__ __forceinline__ void k_update_body(const FieldSet<T> &state, const Fi
     }
 }
 
-template <typename T, int SCHEME, bool STATS = false, bool BATCH = false>
-__global__ void __launch_bounds__(256)
+// FP32: three blocks per SM (80 registers), the viscous factors computed once for u, v, w and the number of fields
+// fixed took the update of 512^3 from 0.419 to 0.346 ms, 256^3 0.066 to 0.054, 128^3 19 to 16.5 us.
+template <typename T, int SCHEME, int NF, bool STATS = false>
+__global__ void __launch_bounds__(256, STATS ? (sizeof(T) == 4 ? 2 : 1) : (sizeof(T) == 4 ? 3 : 2))
 k_update(const __grid_constant__ FieldSet<T> state, const __grid_constant__ FieldSet<T> hist,
          const __grid_constant__ FieldSet<T> nl, Geom g, KeepMap kx_keep, KeepMap ky_keep, int nkz, int ncp,
-         UpdCoef c, int full_rows, double *__restrict__ partial = nullptr, double2 *__restrict__ mean = nullptr) {
-    k_update_body<T, SCHEME, STATS, false>(state, hist, nl, g, kx_keep, ky_keep, nkz, ncp, c, full_rows, partial,
-                                           mean, nullptr, 1, 0, 0);
+         UpdCoef c, int full_rows, double *__restrict__ partial, double2 *__restrict__ mean, int lpr) {
+    k_update_body<T, SCHEME, NF, STATS, false>(state, hist, nl, g, kx_keep, ky_keep, nkz, ncp, c, full_rows, partial,
+                                               mean, nullptr, 1, 0, 0, lpr);
 }
-template <typename T, int SCHEME>
-__global__ void __launch_bounds__(256)
+template <typename T, int SCHEME, int NF>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2)
 k_update_batch(const __grid_constant__ FieldSet<T> state, const __grid_constant__ FieldSet<T> hist,
                const __grid_constant__ FieldSet<T> nl, Geom g, KeepMap kx_keep, KeepMap ky_keep, int nkz, int ncp,
                UpdCoef c, int full_rows, const __grid_constant__ MemberCoef mc, int nmem, long long ms_sh,
-               long long ms_nl) {
-    k_update_body<T, SCHEME, false, true>(state, hist, nl, g, kx_keep, ky_keep, nkz, ncp, c, full_rows, nullptr,
-                                          nullptr, &mc, nmem, ms_sh, ms_nl);
+               long long ms_nl, int lpr) {
+    k_update_body<T, SCHEME, NF, false, true>(state, hist, nl, g, kx_keep, ky_keep, nkz, ncp, c, full_rows, nullptr,
+                                              nullptr, &mc, nmem, ms_sh, ms_nl, lpr);
 }
 
 // ------------------------------------------------------------ statistics
