@@ -536,7 +536,7 @@ struct gnss_server {
     std::deque<Request *> pending;
     std::vector<Request *> active;            // scheduler thread only (sizes read under mu)
     std::map<long long, Request *> reqs;      // every request not yet fetched
-    std::vector<gnss_ctx *> retired;          // contexts of ended requests, destroyed with the server
+    std::deque<gnss_ctx *> retired;           // contexts of ended requests, for requests of the same geometry (mu)
     long long next_id = 1;
     bool stop = false;
     gnss_server_report rep{};
@@ -560,8 +560,57 @@ static void req_release_device(gnss_server *s, Request *r) {
     if (r->stream) cudaStreamDestroy(r->stream);   // returns at once; pending frees still run
     r->ev = nullptr;
     r->stream = nullptr;
-    if (r->ctx) s->retired.push_back(r->ctx);
+    if (r->ctx) {
+        std::lock_guard<std::mutex> lk(s->mu);
+        s->retired.push_back(r->ctx);
+    }
     r->ctx = nullptr;
+}
+
+// Contexts kept for reuse at most; beyond that the one unused for longest is destroyed.
+constexpr size_t RETIRED_MAX = 64;
+
+// A context for a request: one of an ended request of the same geometry, or a new one.
+static gnss_status take_context(gnss_server *s, const gnss_config *cfg, gnss_ctx **out) {
+    gnss_ctx *old = nullptr;
+    {
+        std::lock_guard<std::mutex> lk(s->mu);
+        for (auto it = s->retired.begin(); it != s->retired.end(); ++it)
+            if (gnss_recycle(*it, cfg)) {
+                *out = *it;
+                s->retired.erase(it);
+                return GNSS_OK;
+            }
+        if (s->retired.size() > RETIRED_MAX) {
+            old = s->retired.front();
+            s->retired.pop_front();
+        }
+    }
+    if (old) gnss_destroy(old);
+    return gnss_create(cfg, out);
+}
+
+// Host copy of a state, split over threads when it is large (one core copies at a fraction of the memory's rate, and
+// the pages of a fresh destination are touched for the first time).
+static void copy_state(void *dst, const void *src, size_t bytes) {
+    constexpr size_t PART = 4u << 20;
+    const size_t parts = std::min<size_t>(8, bytes / PART);
+    std::vector<std::thread> th;
+    size_t done = 0;
+    if (parts > 1) {
+        const size_t each = bytes / parts / 4096 * 4096;
+        try {
+            th.reserve(parts);
+            for (size_t i = 0; i + 1 < parts; ++i) {
+                th.emplace_back([=] { std::memcpy(static_cast<char *>(dst) + i * each,
+                                                  static_cast<const char *>(src) + i * each, each); });
+                done += each;
+            }
+        } catch (...) {   // no thread or memory to be had: the rest is copied here
+        }
+    }
+    std::memcpy(static_cast<char *>(dst) + done, static_cast<const char *>(src) + done, bytes - done);
+    for (std::thread &t : th) t.join();
 }
 
 // Upload, dealias and the first step.  Runs on the scheduler thread.
@@ -579,6 +628,7 @@ static gnss_status req_start(Request *r) {
     r->state = fields_at(r->dev, fb, nf);
     r->hist = fields_at(static_cast<char *>(r->dev) + nf * fb, fb, nf);
     gnss_status st = gnss_attach_scratch(r->ctx, r->scratch, r->scratch_bytes);
+    if (!st) st = gnss_reset_run(r->ctx, r->stream);
     if (st) return st;
     if (cudaMemcpyAsync(r->dev, r->h_in, r->state_bytes, cudaMemcpyHostToDevice, r->stream) != cudaSuccess ||
         cudaMemsetAsync(static_cast<char *>(r->dev) + nf * fb, 0, nf * fb, r->stream) != cudaSuccess)
@@ -778,7 +828,7 @@ gnss_status gnss_server_submit(gnss_server *s, const gnss_config *cfg, const voi
     Request *r = new Request;
     r->cfg = *cfg;
     r->n_steps = n_steps;
-    gnss_status st = gnss_create(cfg, &r->ctx);
+    gnss_status st = take_context(s, cfg, &r->ctx);
     if (st) {
         delete r;
         return st;
@@ -797,7 +847,7 @@ gnss_status gnss_server_submit(gnss_server *s, const gnss_config *cfg, const voi
         delete r;
         return GNSS_ERR_NOMEM;
     }
-    std::memcpy(r->h_in, host_state, r->state_bytes);
+    copy_state(r->h_in, host_state, r->state_bytes);
     {
         std::lock_guard<std::mutex> lk(s->mu);
         if (s->stop) {
@@ -840,7 +890,7 @@ gnss_status gnss_server_result(gnss_server *s, long long id, void *host_state_ou
     }
     const gnss_status st = r->status;
     if (st == GNSS_OK) {
-        if (host_state_out) std::memcpy(host_state_out, r->h_out, r->state_bytes);
+        if (host_state_out) copy_state(host_state_out, r->h_out, r->state_bytes);
         if (stats) std::memcpy(stats, r->stats, sizeof r->stats);
     }
     if (times) {

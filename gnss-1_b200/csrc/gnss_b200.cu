@@ -25,13 +25,14 @@ struct gnss_ctx {
     Geom g{};
     size_t nspec = 0;       // complex elements per field
     size_t elem = 0;        // bytes per complex element
+    void *block = nullptr;                        // the context's own device memory (make_device_block)
     void *tw[3] = {nullptr, nullptr, nullptr};   // twiddle tables for nx, ny, nz
     void *scratch = nullptr;                      // nscratch fields
     int nscratch = 0;
     bool scratch_ext = false;                     // scratch attached by the caller (not owned)
     double *stat_part = nullptr;                  // STAT_BLOCKS x STAT_SUMS
     double *stat_dev = nullptr;                   // STAT_SUMS
-    double *stat_host = nullptr;                  // pinned STAT_SUMS
+    double stat_host[STAT_SUMS] = {};             // read back by gnss_stats
     double *turb_part = nullptr;                  // STAT_BLOCKS x TURB_SUMS (gnss_turb_stats)
     double *turb_dev = nullptr;                   // TURB_SUMS + 1 sums, then 5 * ny profile values
     double *turb_host = nullptr;                  // pinned copy of turb_dev
@@ -55,7 +56,6 @@ struct gnss_ctx {
     size_t p_elems = 0, q_elems = 0;
     int zvariant = GNSS_VARIANT_AUTO;             // z kernel choice (gnss_set_option)
     int pvariant = GNSS_VARIANT_AUTO;             // x / y pass kernel choice
-    long long n_sphere = 0;                       // kept-box modes inside the dealiasing sphere
     int n_xin = 0;                                // x-inverse inputs (state fields; s twice with alpha)
     signed char xvar_in[6]{}, xvar_n[6]{}, xvar_mul[6][2]{}, xvar_out[6][2]{};
     signed char yvar_n[MAXF]{}, yvar_mul[MAXF][2]{}, yvar_out[MAXF][2]{};
@@ -65,7 +65,7 @@ struct gnss_ctx {
     unsigned *d_err = nullptr;                    // [0] error word set by bounded waits that time out,
                                                   // [1] wait control (GNSS_OPT_TEST_WAIT; 0 normally)
     int test_wait = 0;                            // GNSS_OPT_TEST_WAIT
-    // tables of the dealiasing sphere for k_passd (make_tables, behind d_err): largest kept |kx| per (kept ky, kz column) and
+    // tables of the dealiasing sphere for k_passd (make_device_block): largest kept |kx| per (kept ky, kz column) and
     // largest kept |ky| per kz column, and the x passes' tiles that lie in the sphere
     short *dtab_x = nullptr, *dtab_y = nullptr;
     int *xlist = nullptr;
@@ -756,6 +756,26 @@ gnss_status gnss_check(gnss_ctx *c, void *stream) {
     return GNSS_OK;
 }
 
+// Modes of the kept box inside the dealiasing sphere (the ones k_update touches after the first step).
+static long long sphere_modes(const gnss_ctx *c) {
+    const Geom &g = c->g;
+    auto wn = [](int i, int n, double dk) { return (i < n / 2) ? dk * (double)i : dk * ((double)i - (double)n); };
+    long long modes = 0;
+    for (int yc = 0; yc < c->ky_keep.count(); ++yc) {
+        const double k2 = wn(c->ky_keep.expand(yc), g.ny, g.dky);
+        for (int xc = 0; xc < c->kx_keep.count(); ++xc) {
+            const double k1 = wn(c->kx_keep.expand(xc), g.nx, g.dkx);
+            const double t = k1 * k1 + k2 * k2;
+            for (int z = 0; z < c->nkz; ++z) {
+                const double k3 = wn(z, g.nz, g.dkz);
+                if (t + k3 * k3 > g.kmax2) break;
+                ++modes;
+            }
+        }
+    }
+    return modes;
+}
+
 gnss_status gnss_stage_bytes(const gnss_ctx *c, double *bytes) {
     if (!c || !bytes) return GNSS_ERR_INVALID;
     const double e = (double)c->elem;
@@ -769,7 +789,7 @@ gnss_status gnss_stage_bytes(const gnss_ctx *c, double *bytes) {
     bytes[2] = e * (c->n_raw * qe + c->nnl * qe);              // z physical
     bytes[3] = e * (c->nnl * qe + c->nnl * pe);                // y forward
     bytes[4] = e * (c->nnl * pe + c->nnl * re);                // x forward
-    const double sph = (double)c->n_sphere;
+    const double sph = (double)sphere_modes(c);
     bytes[5] = e * (c->nnl * sph + 4.0 * nf * sph);            // update (after the first step): nl, state, hist in;
                                                                // state, hist out, inside the sphere
     return GNSS_OK;
@@ -866,22 +886,14 @@ gnss_status gnss_attach_scratch(gnss_ctx *c, void *ptr, size_t bytes) {
     return GNSS_OK;
 }
 
-template <typename T> static void *make_twiddles(int n, gnss_ctx *c) {
-    std::vector<V2<T>> h(n);
+template <typename T> static void fill_twiddles(int n, void *out) {
+    V2<T> *h = static_cast<V2<T> *>(out);
     const long double twopi = 6.283185307179586476925286766559L;
     for (int k = 0; k < n; ++k) {
         long double a = twopi * (long double)k / (long double)n;
         h[k].x = (T)cosl(a);
         h[k].y = (T)(-sinl(a));
     }
-    void *d = nullptr;
-    if (cudaMalloc(&d, sizeof(V2<T>) * n) != cudaSuccess) return nullptr;
-    if (cudaMemcpy(d, h.data(), sizeof(V2<T>) * n, cudaMemcpyHostToDevice) != cudaSuccess) {
-        cudaFree(d);
-        return nullptr;
-    }
-    c->owned_bytes += sizeof(V2<T>) * n;
-    return d;
 }
 
 // Derivatives are split across the passes: kx factors in the x inverse, ky
@@ -992,32 +1004,21 @@ static void set_layout(gnss_ctx *c) {
     c->ncp = (c->nkz + 15) / 16 * 16;
     c->p_elems = (size_t)g.nx * c->ky_keep.count() * c->ncp;
     c->q_elems = (size_t)g.nx * g.ny * c->ncp;
-    // modes of the kept box inside the dealiasing sphere (the ones k_update touches after the first step)
-    auto wn = [](int i, int n, double dk) { return (i < n / 2) ? dk * (double)i : dk * ((double)i - (double)n); };
-    c->n_sphere = 0;
-    for (int yc = 0; yc < c->ky_keep.count(); ++yc) {
-        const double k2 = wn(c->ky_keep.expand(yc), g.ny, g.dky);
-        for (int xc = 0; xc < c->kx_keep.count(); ++xc) {
-            const double k1 = wn(c->kx_keep.expand(xc), g.nx, g.dkx);
-            const double t = k1 * k1 + k2 * k2;
-            for (int z = 0; z < c->nkz; ++z) {
-                const double k3 = wn(z, g.nz, g.dkz);
-                if (t + k3 * k3 > g.kmax2) break;
-                ++c->n_sphere;
-            }
-        }
-    }
 }
 
-// The error words and, behind them in the same allocation, the tables of the
-// dealiasing sphere for k_passd: the kept rows of a column are those whose
-// |index| does not exceed its bound, since k^2 grows with the row's
-// wavenumber; the bounds use the test k^2 > kmax^2 (solver.cu:36) in the
-// reference's order of evaluation.  With both pass lengths on k_passd the x
-// passes visit only the tiles (kept ky, column block) whose first column has a
-// mode inside the sphere, and the y passes leave the rows outside it alone; x
-// tiles are 128 bytes wide (8 FP64 or 16 FP32 columns).
-static gnss_status make_tables(gnss_ctx *c) {
+// What a context keeps on the device, in one allocation filled by one copy
+// (creating a context costs one cudaMalloc and its destruction one cudaFree,
+// which synchronises the device): the error words, the twiddle tables, the
+// FP64 mean-profile line of FP32 contexts (zero: taken from the fields), the
+// tables of the dealiasing sphere for k_passd and the statistics' partial sums.
+// Sphere tables: the kept rows of a column are those whose |index| does not
+// exceed its bound, since k^2 grows with the row's wavenumber; the bounds use
+// the test k^2 > kmax^2 (solver.cu:36) in the reference's order of evaluation.
+// With both pass lengths on k_passd the x passes visit only the tiles (kept
+// ky, column block) whose first column has a mode inside the sphere, and the y
+// passes leave the rows outside it alone; x tiles are 128 bytes wide (8 FP64
+// or 16 FP32 columns).
+static gnss_status make_device_block(gnss_ctx *c) {
     const Geom &g = c->g;
     const int nky = c->ky_keep.count(), ncp = c->ncp, nb = c->elem == sizeof(double2) ? 8 : 16;
     auto wn = [](int i, int n, double dk) { return (i < n / 2) ? dk * (double)i : dk * ((double)i - (double)n); };
@@ -1042,26 +1043,49 @@ static gnss_status make_tables(gnss_ctx *c) {
             r[z] = (short)d;
         }
     }
-    const size_t head = 256, tb = (t.size() * sizeof(short) + 15) / 16 * 16, lb = list.size() * sizeof(int);
-    std::vector<char> h(head + tb + lb, 0);
-    if (!t.empty()) memcpy(h.data() + head, t.data(), t.size() * sizeof(short));
-    if (!list.empty()) memcpy(h.data() + head + tb, list.data(), lb);
-    void *d = nullptr;
-    if (cudaMalloc(&d, h.size()) != cudaSuccess) {
+    size_t bytes = 0;
+    auto part = [&](size_t n) {   // 256-byte aligned
+        const size_t at = bytes;
+        bytes += (n + 255) / 256 * 256;
+        return at;
+    };
+    const int ns[3] = {g.nx, g.ny, g.nz};
+    const size_t at_err = part(2 * sizeof(unsigned));
+    size_t at_tw[3];
+    for (int a = 0; a < 3; ++a) at_tw[a] = part(c->elem * ns[a]);
+    const bool fp32 = c->cfg.precision == GNSS_FP32;
+    const size_t at_mean = part(fp32 ? sizeof(double2) * 10 * (size_t)g.ny : 0);
+    const size_t at_tab = part(t.size() * sizeof(short)), at_list = part(list.size() * sizeof(int));
+    std::vector<char> h(bytes, 0);
+    const size_t at_part = part(sizeof(double) * STAT_BLOCKS * STAT_SUMS), at_stat = part(sizeof(double) * STAT_SUMS);
+    for (int a = 0; a < 3; ++a) {
+        if (fp32) fill_twiddles<float>(ns[a], h.data() + at_tw[a]);
+        else fill_twiddles<double>(ns[a], h.data() + at_tw[a]);
+    }
+    if (!t.empty()) memcpy(h.data() + at_tab, t.data(), t.size() * sizeof(short));
+    if (!list.empty()) memcpy(h.data() + at_list, list.data(), list.size() * sizeof(int));
+    void *dev = nullptr;
+    if (cudaMalloc(&dev, bytes) != cudaSuccess) {
         cudaGetLastError();
         return GNSS_ERR_NOMEM;
     }
-    c->d_err = static_cast<unsigned *>(d);
-    c->owned_bytes += tb + lb;
+    char *d = static_cast<char *>(dev);
+    c->block = dev;
+    c->owned_bytes += bytes;
     if (cudaMemcpy(d, h.data(), h.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
         cudaGetLastError();
         return GNSS_ERR_CUDA;
     }
+    c->d_err = reinterpret_cast<unsigned *>(d + at_err);
+    for (int a = 0; a < 3; ++a) c->tw[a] = d + at_tw[a];
+    if (fp32) c->mean64 = reinterpret_cast<double2 *>(d + at_mean);
+    c->stat_part = reinterpret_cast<double *>(d + at_part);
+    c->stat_dev = reinterpret_cast<double *>(d + at_stat);
     if (!t.empty()) {
-        c->dtab_x = reinterpret_cast<short *>(static_cast<char *>(d) + head);
+        c->dtab_x = reinterpret_cast<short *>(d + at_tab);
         if (pd_size(g.ny)) {
             c->dtab_y = c->dtab_x + (size_t)nky * ncp;
-            c->xlist = reinterpret_cast<int *>(static_cast<char *>(d) + head + tb);
+            c->xlist = reinterpret_cast<int *>(d + at_list);
             c->n_xlist = (int)list.size();
         }
     }
@@ -1098,30 +1122,8 @@ gnss_status gnss_create(const gnss_config *cfg, gnss_ctx **out) {
     c->elem = k.precision == GNSS_FP64 ? sizeof(double2) : sizeof(float2);
     set_recipes(c);
     set_layout(c);
-    const gnss_status tables = make_tables(c);
-    if (tables) { gnss_destroy(c); return tables; }
-    const int ns[3] = {k.nx, k.ny, k.nz};
-    for (int a = 0; a < 3; ++a) {
-        c->tw[a] = k.precision == GNSS_FP64 ? make_twiddles<double>(ns[a], c) : make_twiddles<float>(ns[a], c);
-        if (!c->tw[a]) { gnss_destroy(c); return GNSS_ERR_NOMEM; }
-    }
-    if (cudaMalloc(&c->stat_part, sizeof(double) * STAT_BLOCKS * STAT_SUMS) != cudaSuccess ||
-        cudaMalloc(&c->stat_dev, sizeof(double) * STAT_SUMS) != cudaSuccess ||
-        cudaMallocHost(&c->stat_host, sizeof(double) * STAT_SUMS) != cudaSuccess) {
-        cudaGetLastError();
-        gnss_destroy(c);
-        return GNSS_ERR_NOMEM;
-    }
-    c->owned_bytes += sizeof(double) * (STAT_BLOCKS * STAT_SUMS + STAT_SUMS);
-    if (k.precision == GNSS_FP32) {   // the mean-profile line in FP64 (k_update); zero: taken from the fields
-        const size_t mb = sizeof(double2) * 10 * (size_t)k.ny;
-        if (cudaMalloc(&c->mean64, mb) != cudaSuccess || cudaMemset(c->mean64, 0, mb) != cudaSuccess) {
-            cudaGetLastError();
-            gnss_destroy(c);
-            return GNSS_ERR_NOMEM;
-        }
-        c->owned_bytes += mb;
-    }
+    const gnss_status block = make_device_block(c);
+    if (block) { gnss_destroy(c); return block; }
     if (cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, k.device) != cudaSuccess) {
         cudaGetLastError();
         gnss_destroy(c);
@@ -1131,19 +1133,33 @@ gnss_status gnss_create(const gnss_config *cfg, gnss_ctx **out) {
     return GNSS_OK;
 }
 
+bool gnss_recycle(gnss_ctx *c, const gnss_config *cfg) {
+    const gnss_config &a = c->cfg, &b = *cfg;
+    if (a.nx != b.nx || a.ny != b.ny || a.nz != b.nz || a.lx != b.lx || a.ly != b.ly || a.lz != b.lz ||
+        a.alias_filter != b.alias_filter || a.n_scalars != b.n_scalars || a.scheme != b.scheme ||
+        a.precision != b.precision || a.device != b.device || (a.alpha != 0.0) != (b.alpha != 0.0))
+        return false;
+    if (!(b.re > 0 && b.sc > 0 && b.sc_c > 0 && b.dt > 0)) return false;   // refused by gnss_create
+    c->cfg = b;
+    c->err.clear();
+    c->launches = 0;
+    return true;
+}
+
+gnss_status gnss_reset_run(gnss_ctx *c, void *stream) {
+    if (c->mean64) CK(c, cudaMemsetAsync(c->mean64, 0, sizeof(double2) * 10 * (size_t)c->g.ny, S(stream)));
+    CK(c, cudaMemsetAsync(c->d_err, 0, sizeof(unsigned), S(stream)));
+    return GNSS_OK;
+}
+
 gnss_status gnss_destroy(gnss_ctx *c) {
     if (!c) return GNSS_ERR_INVALID;
     cudaSetDevice(c->cfg.device);
-    for (int a = 0; a < 3; ++a) if (c->tw[a]) cudaFree(c->tw[a]);
+    if (c->block) cudaFree(c->block);
     if (c->scratch && !c->scratch_ext) cudaFree(c->scratch);
-    if (c->stat_part) cudaFree(c->stat_part);
-    if (c->stat_dev) cudaFree(c->stat_dev);
-    if (c->stat_host) cudaFreeHost(c->stat_host);
     if (c->turb_part) cudaFree(c->turb_part);
     if (c->turb_dev) cudaFree(c->turb_dev);
     if (c->turb_host) cudaFreeHost(c->turb_host);
-    if (c->d_err) cudaFree(c->d_err);
-    if (c->mean64) cudaFree(c->mean64);
     if (c->res) cudaFree(c->res);
     if (c->run_sums) cudaFree(c->run_sums);
     if (c->run_sums_host) cudaFreeHost(c->run_sums_host);

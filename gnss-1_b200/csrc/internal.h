@@ -26,3 +26,11 @@ bool gnss_batch_supported(const gnss_ctx *ctx);
 // bit-identical to gnss_step on it alone.
 gnss_status gnss_step_batch(gnss_ctx *const *ctxs, int n, const gnss_fields *state0, const gnss_fields *hist0,
                             size_t member_bytes, void *scratch, size_t scratch_bytes, int euler, void *stream);
+
+// Gives an idle context (no work in flight, no state of its own) to another
+// run: true when `cfg` has the context's geometry, precision, scheme and
+// fields, and its Reynolds and Schmidt numbers, drift, time step and viscosity
+// have been taken over.  gnss_reset_run then clears, in stream order, what the
+// run before left on the device (the FP64 mean line, the error word).
+bool gnss_recycle(gnss_ctx *ctx, const gnss_config *cfg);
+gnss_status gnss_reset_run(gnss_ctx *ctx, void *stream);

@@ -22,7 +22,7 @@
 //   0.36, 192^3 FP32 0.36 -> 0.18 ms.
 //   The dealiasing sphere: rows outside it are not read, tiles outside it are
 //   not visited (21% of the x passes' tiles), and rows no later stage reads
-//   are not stored; the bounds are tables of the context (make_tables).
+//   are not stored; the bounds are tables of the context (make_device_block).
 // A second output of a tile copies the tile again (from L2) rather than hold
 // its 8 elements in registers through the first transform.
 #pragma once
