@@ -174,6 +174,27 @@ template <int S, int G, int Q, int E, typename V> __device__ __forceinline__ voi
     }
 }
 
+// elementwise products of two real lines (x, y)
+__device__ __forceinline__ float2 lmul(float2 a, float2 b) {
+    float2 o;
+    f2_get(f2(a.x, a.y) * f2(b.x, b.y), o.x, o.y);
+    return o;
+}
+__device__ __forceinline__ double2 lmul(double2 a, double2 b) { return double2{a.x * b.x, a.y * b.y}; }
+__device__ __forceinline__ float2 lfma(float2 a, float2 b, float2 c) {
+    float2 o;
+    f2_get(pfma(f2(a.x, a.y), f2(b.x, b.y), f2(c.x, c.y)), o.x, o.y);
+    return o;
+}
+__device__ __forceinline__ double2 lfma(double2 a, double2 b, double2 c) {
+    return double2{a.x * b.x + c.x, a.y * b.y + c.y};
+}
+template <typename V> __device__ __forceinline__ V lneg(V a) { return V{-a.x, -a.y}; }
+// and of one
+__device__ __forceinline__ double lmul(double a, double b) { return a * b; }
+__device__ __forceinline__ double lfma(double a, double b, double c) { return a * b + c; }
+template <> __device__ __forceinline__ double lneg<double>(double a) { return -a; }
+
 template <typename V> __device__ __forceinline__ V shfl_xor_v(V v, int m) {
     return V{__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m)};
 }
@@ -184,41 +205,64 @@ template <typename T, int N> struct ZrScratch {
     __device__ __forceinline__ int operator()(int k1, int i) const { return k1 * ZRCfg<T, N>::S + i; }
 };
 
+// The 32-point DFT across lanes, all E elements of a lane at once, in radix-2
+// steps taken in pairs (4 4 2): of the two twiddles of a pair only a factor
+// i has to be applied between its steps, the rest is one product after them
+// (before them in the reversed flow graph).  zs32_tw: that product's factors
+// W_32^(SIGN e) of the steps 16, 8 and 4, 2.
+template <typename T, int SIGN> struct Zs32 {
+    V2<T> w16, w4;
+    bool i16, i4;
+    __device__ __forceinline__ Zs32(int lane, const V2<T> *w32) {
+        const int b0 = lane & 1, b1 = (lane >> 1) & 1, b2 = (lane >> 2) & 1, b3 = (lane >> 3) & 1, b4 = lane >> 4;
+        w16 = w32[(lane & 7) * (b4 + 2 * b3)];
+        w4 = w32[4 * b0 * (b2 + 2 * b1)];
+        if (SIGN > 0) { w16.y = -w16.y; w4.y = -w4.y; }
+        i16 = b4 && b3;
+        i4 = b2 && b1;
+    }
+};
+// p + x on the lanes without bit h, p - x on those with it (p: the partner's value)
+template <typename T> __device__ __forceinline__ V2<T> zs_step(int lane, V2<T> x, int h) {
+    const T s = (lane & h) ? T(-1) : T(1);
+    return lfma(V2<T>{s, s}, x, shfl_xor_v(x, h));
+}
+
 // Length-N DFT (N = 32 E, E = 2, 3, 4, 6) of one line held by a warp, with
 // lane shuffles only.  On entry x[m] is element lane + 32 m; on return x[q]
 // is element q + E bitrev5(lane) of the transform.  n = lane + 32 m,
 // k = k1 + E k2: an E-point DFT over m in registers, the twiddle
-// W_N^(lane k1), then for every k1 a 32-point DFT across the lanes in five
-// radix-2 decimation-in-frequency steps (partner lane ^ h: p + s x with s = +1
-// on the lower and -1 on the upper lane, the upper one then multiplied by
-// W_{2h}^(lane mod h)).  tws rows: W_N^(lane k1), k1 = 1 .. E-1, then W_32^lane
-// (exp(-2 pi i ./.), conjugated for SIGN > 0).
+// W_N^(lane k1), then for every k1 a 32-point DFT across the lanes
+// (decimation in frequency).  tws rows: W_N^(lane k1), k1 = 1 .. E-1, then
+// W_32^lane (exp(-2 pi i ./.), conjugated for SIGN > 0).
 template <typename T, int N, int SIGN>
 __device__ __forceinline__ void zs_fft(int lane, V2<T> *x, const V2<T> *tws) {
     using V = V2<T>;
     constexpr int E = N / 32;
-    auto tw_at = [&](int i) {
-        V t = tws[i];
-        if (SIGN > 0) t.y = -t.y;
-        return t;
-    };
     Dft<E, SIGN, V>::run(x);
 #pragma unroll
-    for (int k1 = 1; k1 < E; ++k1) x[k1] = cmul(x[k1], tw_at(32 * (k1 - 1) + lane));
-#pragma unroll
-    for (int h = 16; h >= 1; h >>= 1) {
-        const bool upper = (lane & h) != 0;
-        const T sg = upper ? T(-1) : T(1);
-        V w = V{T(1), T(0)};
-        if (h > 1 && upper) w = tw_at(32 * (E - 1) + (lane & (h - 1)) * (16 / h));
-#pragma unroll
-        for (int q = 0; q < E; ++q) {
-            const V p = shfl_xor_v(x[q], h);
-            V t = V{p.x + sg * x[q].x, p.y + sg * x[q].y};
-            if (h > 1) t = cmul(t, w);
-            x[q] = t;
-        }
+    for (int k1 = 1; k1 < E; ++k1) {
+        V t = tws[32 * (k1 - 1) + lane];
+        if (SIGN > 0) t.y = -t.y;
+        x[k1] = cmul(x[k1], t);
     }
+    const Zs32<T, SIGN> z(lane, tws + 32 * (E - 1));
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+        x[q] = zs_step<T>(lane, x[q], 16);
+        if (z.i16) x[q] = mul_si<SIGN>(x[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < E; ++q) x[q] = cmul(zs_step<T>(lane, x[q], 8), z.w16);
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+        x[q] = zs_step<T>(lane, x[q], 4);
+        if (z.i4) x[q] = mul_si<SIGN>(x[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < E; ++q) x[q] = cmul(zs_step<T>(lane, x[q], 2), z.w4);
+#pragma unroll
+    for (int q = 0; q < E; ++q) x[q] = zs_step<T>(lane, x[q], 1);
 }
 
 // x[k1] *= W_N^(SIGN lane k1), the step-A twiddles of zr_fft (transpose scheme)
@@ -324,28 +368,31 @@ __device__ __forceinline__ void zr_fft_rev(int lane, V2<T> *x, V2<T> *scr, const
     using V = V2<T>;
     using Z = ZRCfg<T, N>;
     constexpr int E = Z::E, G = Z::G;
-    if constexpr (Z::SHFL) {   // the 32-point DFT across lanes: bit-reversed input, decimation in time
+    if constexpr (Z::SHFL) {   // the reverse of zs_fft: bit-reversed input, decimation in time
         (void)scr;
-        auto tw_at = [&](int i) {
-            V t = tws[i];
-            if (SIGN > 0) t.y = -t.y;
-            return t;
-        };
+        const Zs32<T, SIGN> z(lane, tws + 32 * (E - 1));
 #pragma unroll
-        for (int h = 1; h <= 16; h <<= 1) {
-            const bool upper = (lane & h) != 0;
-            const T sg = upper ? T(-1) : T(1);
-            V w = V{T(1), T(0)};
-            if (h > 1 && upper) w = tw_at(32 * (E - 1) + (lane & (h - 1)) * (16 / h));
+        for (int q = 0; q < E; ++q) x[q] = cmul(zs_step<T>(lane, x[q], 1), z.w4);
 #pragma unroll
-            for (int q = 0; q < E; ++q) {
-                const V t = h > 1 ? cmul(x[q], w) : x[q];
-                const V p = shfl_xor_v(t, h);
-                x[q] = V{p.x + sg * t.x, p.y + sg * t.y};
-            }
+        for (int q = 0; q < E; ++q) {
+            x[q] = zs_step<T>(lane, x[q], 2);
+            if (z.i4) x[q] = mul_si<SIGN>(x[q]);
         }
 #pragma unroll
-        for (int k1 = 1; k1 < E; ++k1) x[k1] = cmul(x[k1], tw_at(32 * (k1 - 1) + lane));
+        for (int q = 0; q < E; ++q) x[q] = cmul(zs_step<T>(lane, x[q], 4), z.w16);
+#pragma unroll
+        for (int q = 0; q < E; ++q) {
+            x[q] = zs_step<T>(lane, x[q], 8);
+            if (z.i16) x[q] = mul_si<SIGN>(x[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < E; ++q) x[q] = zs_step<T>(lane, x[q], 16);
+#pragma unroll
+        for (int k1 = 1; k1 < E; ++k1) {
+            V t = tws[32 * (k1 - 1) + lane];
+            if (SIGN > 0) t.y = -t.y;
+            x[k1] = cmul(x[k1], t);
+        }
     } else {
         const int k1 = lane / G, j = lane % G;
         if constexpr (G == 2) {
@@ -485,27 +532,6 @@ __device__ __forceinline__ void zl_unpack(int lane, const V2<T> *x, V2<T> *d, in
     }
     for (int k = lane + 32 * (E / 2 + 1); k < ncp; k += 32) d[k] = d[ncp + k] = V{T(0), T(0)};   // padding of short lines
 }
-
-// elementwise products of two real lines (x, y)
-__device__ __forceinline__ float2 lmul(float2 a, float2 b) {
-    float2 o;
-    f2_get(f2(a.x, a.y) * f2(b.x, b.y), o.x, o.y);
-    return o;
-}
-__device__ __forceinline__ double2 lmul(double2 a, double2 b) { return double2{a.x * b.x, a.y * b.y}; }
-__device__ __forceinline__ float2 lfma(float2 a, float2 b, float2 c) {
-    float2 o;
-    f2_get(pfma(f2(a.x, a.y), f2(b.x, b.y), f2(c.x, c.y)), o.x, o.y);
-    return o;
-}
-__device__ __forceinline__ double2 lfma(double2 a, double2 b, double2 c) {
-    return double2{a.x * b.x + c.x, a.y * b.y + c.y};
-}
-template <typename V> __device__ __forceinline__ V lneg(V a) { return V{-a.x, -a.y}; }
-// and of one
-__device__ __forceinline__ double lmul(double a, double b) { return a * b; }
-__device__ __forceinline__ double lfma(double a, double b, double c) { return a * b + c; }
-template <> __device__ __forceinline__ double lneg<double>(double a) { return -a; }
 
 // Physical lines and their products.  A warp leaves a physical line in shared
 // memory where its transform ends: element zr_out_index(lane, q) at
