@@ -756,24 +756,35 @@ gnss_status gnss_check(gnss_ctx *c, void *stream) {
     return GNSS_OK;
 }
 
-// Modes of the kept box inside the dealiasing sphere (the ones k_update touches after the first step).
-static long long sphere_modes(const gnss_ctx *c) {
+// What of the kept box lies inside the dealiasing sphere: modes (the ones k_update touches after the first step);
+// columns (ky, kz) with a kept mode, and those of the x passes' tiles; modes the x forward pass stores (all columns of
+// a tile with the rows of its first one).
+struct SphereCount {
+    double modes = 0, cols = 0, tile_cols = 0, stored = 0;
+};
+static SphereCount count_sphere(const gnss_ctx *c) {
     const Geom &g = c->g;
+    const int nb = c->elem == sizeof(double2) ? 8 : 16;
     auto wn = [](int i, int n, double dk) { return (i < n / 2) ? dk * (double)i : dk * ((double)i - (double)n); };
-    long long modes = 0;
+    SphereCount n;
     for (int yc = 0; yc < c->ky_keep.count(); ++yc) {
         const double k2 = wn(c->ky_keep.expand(yc), g.ny, g.dky);
-        for (int xc = 0; xc < c->kx_keep.count(); ++xc) {
-            const double k1 = wn(c->kx_keep.expand(xc), g.nx, g.dkx);
-            const double t = k1 * k1 + k2 * k2;
-            for (int z = 0; z < c->nkz; ++z) {
-                const double k3 = wn(z, g.nz, g.dkz);
-                if (t + k3 * k3 > g.kmax2) break;
-                ++modes;
+        for (int z = 0; z < c->nkz; ++z) {
+            const double k3 = wn(z, g.nz, g.dkz);
+            int rows = 0;
+            for (int xc = 0; xc < c->kx_keep.count(); ++xc) {
+                const double k1 = wn(c->kx_keep.expand(xc), g.nx, g.dkx);
+                rows += (k1 * k1 + k2 * k2) + k3 * k3 > g.kmax2 ? 0 : 1;
+            }
+            n.modes += rows;
+            n.cols += rows > 0;
+            if (z % nb == 0 && rows > 0) {
+                n.tile_cols += nb;
+                n.stored += (double)nb * rows;
             }
         }
     }
-    return modes;
+    return n;
 }
 
 gnss_status gnss_stage_bytes(const gnss_ctx *c, double *bytes) {
@@ -781,17 +792,21 @@ gnss_status gnss_stage_bytes(const gnss_ctx *c, double *bytes) {
     const double e = (double)c->elem;
     const int nf = 3 + c->cfg.n_scalars;
     const double nkx = c->kx_keep.count(), nky = c->ky_keep.count();
-    const double box = nky * nkx * c->nkz;                    // kept modes of one state field
-    const double pe = (double)c->p_elems, qe = (double)c->q_elems;
-    const double re = nky * nkx * c->ncp;                     // x-forward output
-    bytes[0] = e * (c->n_xin * box + c->n_xout * pe);          // x inverse
-    bytes[1] = e * (c->n_xout * pe + c->n_raw * qe);           // y inverse
-    bytes[2] = e * (c->n_raw * qe + c->nnl * qe);              // z physical
-    bytes[3] = e * (c->nnl * qe + c->nnl * pe);                // y forward
-    bytes[4] = e * (c->nnl * pe + c->nnl * re);                // x forward
-    const double sph = (double)sphere_modes(c);
-    bytes[5] = e * (c->nnl * sph + 4.0 * nf * sph);            // update (after the first step): nl, state, hist in;
-                                                               // state, hist out, inside the sphere
+    const SphereCount n = count_sphere(c);
+    // the x / y intermediates hold what lies in the sphere (both passes on k_passd), or the whole kept box
+    const bool sphere = c->xlist && (c->pvariant == GNSS_VARIANT_AUTO || c->pvariant == GNSS_VARIANT_REGISTER);
+    const double pw = sphere ? (double)c->g.nx * n.tile_cols : (double)c->p_elems;   // P as its tiles are stored
+    const double pr = sphere ? (double)c->g.nx * n.cols : (double)c->p_elems;        // P as the y inverse reads it
+    const double in = sphere ? n.modes : nky * nkx * c->nkz;                          // modes of one state field read
+    const double re = sphere ? n.stored : nky * nkx * c->ncp;                         // x-forward output
+    const double qe = (double)c->q_elems;
+    bytes[0] = e * (c->n_xin * in + c->n_xout * pw);            // x inverse
+    bytes[1] = e * (c->n_xout * pr + c->n_raw * qe);            // y inverse
+    bytes[2] = e * (c->n_raw * qe + c->nnl * qe);               // z physical
+    bytes[3] = e * (c->nnl * qe + c->nnl * pw);                 // y forward
+    bytes[4] = e * (c->nnl * pw + c->nnl * re);                 // x forward
+    bytes[5] = e * (c->nnl * n.modes + 4.0 * nf * n.modes);     // update (after the first step): nl, state, hist in;
+                                                                // state, hist out, inside the sphere
     return GNSS_OK;
 }
 
