@@ -12,8 +12,8 @@ constexpr int GNSS_BATCH_MAX = 16;
 // intermediates of the context's geometry).
 size_t gnss_batch_scratch_bytes(const gnss_ctx *ctx);
 
-// Whether a context's kernel choices allow batched steps: the register z
-// kernel and x / y lengths with register passes (64 .. 512).
+// Whether a context's kernel choices allow batched steps: the CN/AB2 scheme,
+// GNSS_OPT_ZKERNEL == GNSS_VARIANT_REGISTER, and x / y lengths of zr_size().
 bool gnss_batch_supported(const gnss_ctx *ctx);
 
 // One fused step of n members of one geometry (grid, precision, scalar count,

@@ -107,6 +107,8 @@ template <typename T, int N> struct PassLaunch {
     }
     static cudaError_t zpass(int dir, const FieldSet<T> &f, int nfields, long long nlines, int nz2, T scale,
                              const void *tw, cudaStream_t s) {
+        // register transforms at every length they serve (192 x 256 x 128 FP64, forward + inverse with all passes:
+        // 241 us with k_zpass, 202 with k_zline)
         if constexpr (zr_size(N)) {
             using Z = ZRCfg<T, N>;
             const int smem = (Z::LOGE * 32 + ZLINE_WARPS * Z::SCR) * (int)sizeof(V2<T>);

@@ -1,7 +1,7 @@
 // passtc.cuh -- strided x / y passes whose line transforms run on the tensor
 // cores as split-TF32 DFT-matrix GEMMs (FP32, N = 256 and 512).
 //
-// Same contract as k_passr / k_pass (PassSpec / PassPtrs: tiles of columns x N
+// Same contract as k_pass (PassSpec / PassPtrs: tiles of columns x N
 // rows, kept / compact rows and outer indices, up to two outputs per tile,
 // each the transform of the tile times a spectral multiplier, optional dealias
 // mask), for tiles of NB = 8 columns.  A length-N transform, N = N1 N2 with

@@ -555,8 +555,11 @@ template <typename T, int N> __host__ __device__ constexpr int zl_stride() {
 // place.  Modes go between global memory and registers, points through a
 // shared line, so that both sides are coalesced.  A field has an even number
 // of lines.
-//   Measured against k_zpass (a shared-memory round trip per radix-8 stage):
-// see the launcher.
+//   Bound by HBM and by how many lines are in flight: a warp holds one pair at
+// a time, so four warps per block and as many blocks as fit keep loads going
+// while others transform.  Measured against k_zpass (a shared-memory round trip
+// per radix-8 stage), forward + inverse of a 192 x 256 x 128 FP64 field, all
+// six passes: 241 -> 202 us.
 constexpr int ZLINE_WARPS = 4;
 template <typename T, int N, int DIR>
 __global__ void __launch_bounds__(ZLINE_WARPS * 32)

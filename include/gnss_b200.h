@@ -240,22 +240,23 @@ gnss_status gnss_profile_read(gnss_ctx *ctx, double *ms, long long *launches);
  * GNSS_OPT_ZVARIANT picks the kernel of the fused z stage, GNSS_OPT_PVARIANT
  * the kernel of the strided x and y passes (of the step and of the 3D
  * transforms):
- *   GNSS_VARIANT_AUTO      the kernel measured fastest on B200: register-
- *                          resident transforms where they fit (z: every N
- *                          below, with separate inverse and forward warps
- *                          in FP64 where that kernel exists; x / y passes:
- *                          N = 96 .. 512 in FP32, 256 and 512 in FP64),
+ *   GNSS_VARIANT_AUTO      the kernel measured fastest on B200: the
+ *                          register kernels at every length they serve,
  *                          staged otherwise;
- *   GNSS_VARIANT_REGISTER  register-resident transforms where they exist
- *                          (N = 64, 96, 128, 192 with lane shuffles only;
- *                          N = 256, 512 with one transpose) and fit (a
- *                          request, not a guarantee);
- *   GNSS_VARIANT_STAGED    per-radix-stage transforms through shared memory;
- *   GNSS_VARIANT_WARPSPEC  (GNSS_OPT_ZVARIANT only) the register z kernel
- *                          with separate inverse and forward warps, where it
- *                          exists (z length 256 or 512, no colloid term; FP32
- *                          with one scalar, FP64 with one or two); the
- *                          register kernel otherwise;
+ *   GNSS_VARIANT_REGISTER  the register kernels where they exist and fit (a
+ *                          request, not a guarantee).  z lengths 64, 96,
+ *                          128, 192, 256, 512: one warp per line pair of one
+ *                          quantity, separate inverse and forward warps.
+ *                          x / y lengths 48, 64, 96, 128, 192, 256, 384,
+ *                          512: radix-8 columns, 8 elements per thread; with
+ *                          both lengths among them the intermediates are
+ *                          confined to the dealiasing sphere;
+ *   GNSS_VARIANT_STAGED    per-radix-stage transforms through shared memory,
+ *                          over the whole kept box;
+ *   GNSS_VARIANT_WARPSPEC  (GNSS_OPT_ZVARIANT only) another name for the
+ *                          register z kernel; GNSS_OPT_ZKERNEL reports it at
+ *                          z lengths 256 and 512 without the colloid term
+ *                          (FP32 with one scalar, FP64 with one or two);
  *   GNSS_VARIANT_TENSOR    (GNSS_OPT_PVARIANT only) line transforms on the
  *                          tensor cores as split-TF32 DFT-matrix GEMMs
  *                          (tcgen05, three TF32 products per GEMM with FP32
@@ -343,7 +344,7 @@ int gnss_ensemble_batched(const gnss_ensemble *e, int i);
  * branch streams and, where the kernels allow it, as batched launches, on the
  * members' own buffers (which are zeroed afterwards, so tune before uploading
  * states), and keep the fastest form with the fastest of the z variants
- * REGISTER, STAGED, WARPSPEC by the pass variants REGISTER, STAGED and, where
+ * REGISTER, STAGED by the pass variants REGISTER, STAGED and, where
  * it exists (FP32, an x or y length of 256 or 512), TENSOR.  choices (may be
  * NULL) receives, per member, the chosen GNSS_OPT_ZVARIANT value + 4 * the
  * GNSS_OPT_PVARIANT value; gnss_ensemble_batched reports the form. */
