@@ -501,7 +501,7 @@ static gnss_status nonlinear_and_update(gnss_ctx *c, const gnss_fields *state, v
             CK(c, launch_dep(ku, dim3((unsigned)nblk), dim3(256), 0, s, SF, H, R, g, c->kx_keep, c->ky_keep, c->nkz,
                              c->ncp, uc, full_rows, c->stat_part, c->mean64, lpr));
             c->launches++;
-            CK(c, launch_dep(k_stats_final, dim3(1), dim3(STAT_SUMS * 32), 0, s, (const double *)c->stat_part,
+            CK(c, launch_dep(k_stats_final, dim3(1), dim3(STATS_FINAL_THREADS), 0, s, (const double *)c->stat_part,
                              (int)nblk, stats_dst));
             return GNSS_OK;
         }
@@ -564,9 +564,9 @@ template <typename T> static gnss_status stats_t(gnss_ctx *c, const gnss_fields 
     for (int q = 0; q < 5; ++q) F.p[q] = reinterpret_cast<V2<T> *>(sp[q]);
     const int has_s = st->s != nullptr, has_c = st->c != nullptr;
     c->launches += 2;
-    k_stats_partial<T><<<STAT_BLOCKS, STAT_THREADS, 0, s>>>(F, has_s, has_c, c->g, c->stat_part);
+    k_stats_partial<T><<<WALK_BLOCKS, STAT_THREADS, 0, s>>>(F, has_s, has_c, c->g, c->stat_part);
     LAUNCH_CK(c);
-    k_stats_final<<<1, STAT_SUMS * 32, 0, s>>>(c->stat_part, STAT_BLOCKS, c->stat_dev);
+    k_stats_final<<<1, STATS_FINAL_THREADS, 0, s>>>(c->stat_part, WALK_BLOCKS, c->stat_dev);
     LAUNCH_CK(c);
     CK(c, cudaMemcpyAsync(c->stat_host, c->stat_dev, sizeof(double) * STAT_SUMS, cudaMemcpyDeviceToHost, s));
     CK(c, cudaStreamSynchronize(s));
@@ -613,11 +613,11 @@ static gnss_status ensure_turb_buffers(gnss_ctx *c) {
 template <typename T> static gnss_status turb_spectral_t(gnss_ctx *c, const FieldSet<T> &F, bool has_s, cudaStream_t s) {
     const Geom &g = c->g;
     c->launches += 3;
-    k_turb_partial<T><<<STAT_BLOCKS, STAT_THREADS, 0, s>>>(F, has_s, g, c->turb_part);
+    k_turb_partial<T><<<WALK_BLOCKS, STAT_THREADS, 0, s>>>(F, has_s, g, c->turb_part);
     LAUNCH_CK(c);
-    k_sums_final<TURB_SUMS><<<1, TURB_SUMS * 32, 0, s>>>(c->turb_part, STAT_BLOCKS, TURB_SUMS, c->turb_dev);
+    k_sums_final<TURB_SUMS><<<1, TURB_SUMS * FINAL_WARPS * 32, 0, s>>>(c->turb_part, WALK_BLOCKS, c->turb_dev);
     LAUNCH_CK(c);
-    k_yprof<T><<<5, 256, 0, s>>>(F, g, reinterpret_cast<const V2<T> *>(c->tw[1]),
+    k_yprof<T><<<dim3(5, (g.ny + YPROF_THREADS - 1) / YPROF_THREADS), YPROF_THREADS, 0, s>>>(F, g, reinterpret_cast<const V2<T> *>(c->tw[1]),
                                  c->turb_dev + TURB_SUMS + VORT_SUMS);
     LAUNCH_CK(c);
     return GNSS_OK;
@@ -642,7 +642,7 @@ template <typename T> static gnss_status turb_vort_t(gnss_ctx *c, const FieldSet
                                                             reinterpret_cast<const T *>(o[1]),
                                                             reinterpret_cast<const T *>(o[2]), g, c->turb_part);
     LAUNCH_CK(c);
-    k_sums_final<VORT_SUMS><<<1, VORT_SUMS * 32, 0, s>>>(c->turb_part, STAT_BLOCKS, VORT_SUMS,
+    k_sums_final<VORT_SUMS><<<1, VORT_SUMS * FINAL_WARPS * 32, 0, s>>>(c->turb_part, STAT_BLOCKS,
                                                          c->turb_dev + TURB_SUMS);
     LAUNCH_CK(c);
     return GNSS_OK;
@@ -712,7 +712,7 @@ static gnss_status step_turb_t(gnss_ctx *c, const gnss_fields *st, const gnss_fi
         CK(c, cudaMemsetAsync(c->turb_part, 0, sizeof(double) * STAT_BLOCKS * VORT_SUMS, s));
         if ((r = step_t<T>(c, st, hist, euler, s, nullptr, c->turb_part))) return r;
         c->launches++;
-        k_sums_final<VORT_SUMS><<<1, VORT_SUMS * 32, 0, s>>>(c->turb_part, STAT_BLOCKS, VORT_SUMS,
+        k_sums_final<VORT_SUMS><<<1, VORT_SUMS * FINAL_WARPS * 32, 0, s>>>(c->turb_part, STAT_BLOCKS,
                                                              c->turb_dev + TURB_SUMS);
         LAUNCH_CK(c);
     } else {

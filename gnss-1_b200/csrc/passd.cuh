@@ -11,7 +11,7 @@
 // to global memory.  Eight elements per thread keep it at 80 registers, 24
 // warps per SM (16 at N = 512, whose two tiles fill an SM's shared memory).
 //   What bounds it: instruction issue and shared-memory wavefronts (ncu, 512
-//   rows: LSU wavefronts 59% FP64, 48% FP32, issue 41 / 47%), so what is fixed
+//   rows: LSU wavefronts 54-59% FP64, 53-56% FP32, issue 40 / 45%), so what is fixed
 //   for the launch stays out of the loop: the rows a thread reads and stores
 //   as bit masks, work items advanced by the grid size instead of divided,
 //   two base pointers (lower and upper half of the rows: the gap of a compact

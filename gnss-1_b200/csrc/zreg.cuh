@@ -621,9 +621,10 @@ template <typename T, int NPH> __device__ __forceinline__ T zr_line_scale(int q,
 // Product f at this lane's points: (w x u)_f (crossProductKernel_mgpu,
 // solver.cu:139-164) for f < 3, u . grad s (dotKernel_mgpu, solver.cu:342-356)
 // for 3, u . grad c and the colloid term (colloidAdvectionKernel_mgpu,
-// solver.cu:374-388) for 4.  With DIAG the warp of product 0 also adds the
-// vorticity sums of its points to acc (ZR_VORT_SUMS: |w|, w_x^2, w_y^2, w_z^2,
-// both lines; statistics.cu:1211-1305).
+// solver.cu:374-388) for 4.  With DIAG each of the first four warps
+// also adds the vorticity sums of a quarter of the points to acc
+// (ZR_VORT_SUMS: |w|, w_x^2, w_y^2, w_z^2, both lines;
+// statistics.cu:1211-1305).
 constexpr int ZR_VORT_SUMS = 4;
 template <typename T, int N, int NPH, bool DIAG>
 __device__ __forceinline__ void zl_product(int f, int lane, V2<T> *x, const V2<T> *lines, T alpha, T scale, double *acc) {
@@ -631,26 +632,24 @@ __device__ __forceinline__ void zl_product(int f, int lane, V2<T> *x, const V2<T
     using Z = ZRCfg<T, N>;
     constexpr int E = Z::E, ST = zl_stride<T, N>(), L = Z::SCR;
     const V *p = lines + zl_base<T, N>(lane);
+    if constexpr (DIAG) {   // the FP64 sums shared out: with one warp on all of them the others
+        // waited for it (256^3 FP32 432 us against 331, 325 without the sums)
+        const double s = zr_fold_scale<NPH>() ? (double)scale : 1.0;
+        for (int q = f; q < (f < 4 ? E : 0); q += 4) {
+            const V w1 = p[3 * L + q * ST], w2 = p[4 * L + q * ST], w3 = p[5 * L + q * ST];
+            const double ax = s * w1.x, ay = s * w2.x, az = s * w3.x, bx = s * w1.y, by = s * w2.y, bz = s * w3.y;
+            acc[0] += sqrt(ax * ax + ay * ay + az * az) + sqrt(bx * bx + by * by + bz * bz);
+            acc[1] += ax * ax + bx * bx;
+            acc[2] += ay * ay + by * by;
+            acc[3] += az * az + bz * bz;
+        }
+    }
     if (f < 3) {
         // w2 w - w3 v, w3 u - w1 w, w1 v - w2 u
         const V *a = p + (f == 2 ? 3 : f + 4) * L, *b = p + (f == 0 ? 2 : f - 1) * L;
         const V *c = p + (f == 0 ? 5 : f + 2) * L, *d = p + (f == 0 ? 1 : f == 1 ? 2 : 0) * L;
 #pragma unroll
         for (int q = 0; q < E; ++q) x[q] = lfma(a[q * ST], b[q * ST], lneg(lmul(c[q * ST], d[q * ST])));
-        if constexpr (DIAG) {
-            if (f == 0) {
-                const double s = zr_fold_scale<NPH>() ? (double)scale : 1.0;
-#pragma unroll
-                for (int q = 0; q < E; ++q) {
-                    const V w1 = p[3 * L + q * ST], w2 = p[4 * L + q * ST], w3 = p[5 * L + q * ST];
-                    const double ax = s * w1.x, ay = s * w2.x, az = s * w3.x, bx = s * w1.y, by = s * w2.y, bz = s * w3.y;
-                    acc[0] += sqrt(ax * ax + ay * ay + az * az) + sqrt(bx * bx + by * by + bz * bz);
-                    acc[1] += ax * ax + bx * bx;
-                    acc[2] += ay * ay + by * by;
-                    acc[3] += az * az + bz * bz;
-                }
-            }
-        }
     } else {
         const V *g = p + (f == 3 ? 6 : 9) * L;
 #pragma unroll
@@ -798,14 +797,20 @@ k_zpipe(const __grid_constant__ FieldSet<T> f, const __grid_constant__ ZRecipeSe
             end_b();
         }
     }
-    if constexpr (DIAG) {   // the sums lie in the lanes of one warp: added in a fixed order
-        if (warp == NPH) {
+    if constexpr (DIAG) {   // the sums lie in the lanes of four warps: added in a fixed order
+        __shared__ double red[ZR_VORT_SUMS][4];
+        if (warp >= NPH && warp < NPH + 4) {
 #pragma unroll
             for (int q = 0; q < ZR_VORT_SUMS; ++q) {
                 double v = acc[q];
                 for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-                if (lane == 0) diag[blockIdx.x * ZR_VORT_SUMS + q] = v;
+                if (lane == 0) red[q][warp - NPH] = v;
             }
+        }
+        __syncthreads();
+        if (threadIdx.x < ZR_VORT_SUMS) {
+            const double *r = red[threadIdx.x];
+            diag[blockIdx.x * ZR_VORT_SUMS + threadIdx.x] = ((r[0] + r[1]) + r[2]) + r[3];
         }
     }
 }
