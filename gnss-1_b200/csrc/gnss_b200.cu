@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "gnss_b200.h"
+#include "hostblock.h"
 #include "internal.h"
 #include "launch.h"
 #include "diag.cuh"
@@ -816,7 +817,7 @@ gnss_status gnss_set_option(gnss_ctx *c, int key, int value) {
         if (value < 0) return fail(c, GNSS_ERR_INVALID, "bad poll cap %d", value);
         CK(c, cudaSetDevice(c->cfg.device));
         const unsigned v = (unsigned)value;
-        CK(c, cudaMemcpy(c->d_err + 1, &v, sizeof v, cudaMemcpyHostToDevice));
+        CK(c, upload_and_wait(c->d_err + 1, &v, sizeof v));
         c->test_wait = value;
         return GNSS_OK;
     }
@@ -1087,7 +1088,7 @@ static gnss_status make_device_block(gnss_ctx *c) {
     char *d = static_cast<char *>(dev);
     c->block = dev;
     c->owned_bytes += bytes;
-    if (cudaMemcpy(d, h.data(), h.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (upload_and_wait(d, h.data(), h.size()) != cudaSuccess) {
         cudaGetLastError();
         return GNSS_ERR_CUDA;
     }
