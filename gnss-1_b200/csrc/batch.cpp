@@ -536,7 +536,8 @@ struct gnss_server {
     std::deque<Request *> pending;
     std::vector<Request *> active;            // scheduler thread only (sizes read under mu)
     std::map<long long, Request *> reqs;      // every request not yet fetched
-    std::deque<gnss_ctx *> retired;           // contexts of ended requests, for requests of the same geometry (mu)
+    std::deque<gnss_ctx *> retired;           // idle contexts of ended requests, for requests of the same geometry (mu)
+    std::vector<gnss_ctx *> spent;            // contexts not offered again, destroyed with the server (mu)
     long long next_id = 1;
     bool stop = false;
     gnss_server_report rep{};
@@ -548,7 +549,11 @@ static double now_s(const gnss_server *s) {
     return std::chrono::duration<double>(Clock::now() - s->t0).count();
 }
 
+// A request that ended well has an idle context (its last event has completed), which may serve another request.  One
+// that failed may have left work queued on its stream: that is waited for, and the context is not offered again.
 static void req_release_device(gnss_server *s, Request *r) {
+    const bool idle = r->status == GNSS_OK;
+    if (!idle && r->stream) cudaStreamSynchronize(r->stream);
     if (r->gexec) {
         cudaGraphExecDestroy(r->gexec);
         r->gexec = nullptr;
@@ -562,7 +567,8 @@ static void req_release_device(gnss_server *s, Request *r) {
     r->stream = nullptr;
     if (r->ctx) {
         std::lock_guard<std::mutex> lk(s->mu);
-        s->retired.push_back(r->ctx);
+        if (idle) s->retired.push_back(r->ctx);
+        else s->spent.push_back(r->ctx);
     }
     r->ctx = nullptr;
 }
@@ -811,6 +817,7 @@ gnss_status gnss_server_destroy(gnss_server *s) {
     cudaSetDevice(s->cfg.device);
     cudaDeviceSynchronize();
     for (gnss_ctx *c : s->retired) gnss_destroy(c);
+    for (gnss_ctx *c : s->spent) gnss_destroy(c);
     for (auto &kv : s->reqs) {
         Request *r = kv.second;
         if (r->ctx) gnss_destroy(r->ctx);

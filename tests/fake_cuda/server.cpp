@@ -1,0 +1,71 @@
+// The server of batch.cpp on the host runtime: one scenario per run, named by
+// the first argument.
+#include <cstdio>
+#include <cstring>
+#include <string>
+#include <vector>
+
+#include "fake_ctx.h"
+#include "fake_cuda.h"
+
+#define EXPECT(x)                                             \
+    do {                                                      \
+        if (!(x)) {                                           \
+            std::printf("line %d: %s\n", __LINE__, #x);       \
+            return 1;                                         \
+        }                                                     \
+    } while (0)
+
+static gnss_config config(int n, int device = 0) {
+    gnss_config c{};
+    c.nx = c.ny = c.nz = n;
+    c.n_scalars = 1;
+    c.precision = GNSS_FP32;
+    c.device = device;
+    return c;
+}
+static std::vector<char> state_of(const gnss_config &c) {
+    return std::vector<char>((size_t)c.nx * c.ny * (c.nz / 2 + 1) * 8 * (3 + c.n_scalars), 1);
+}
+static gnss_server *server(int max_active, int device = 0) {
+    gnss_server_config sc{};
+    sc.budget_bytes = (size_t)1 << 34;
+    sc.max_active = max_active;
+    sc.steps_per_launch = 100;   // requests below: single launches
+    sc.device = device;
+    gnss_server *s = nullptr;
+    return gnss_server_create(&sc, &s) == GNSS_OK ? s : nullptr;
+}
+
+// A request whose fourth step fails leaves three steps queued on its stream; its context must not serve another
+// request.
+static int failed_request() {
+    const gnss_config c = config(8);
+    const std::vector<char> st = state_of(c);
+    gnss_server *s = server(4);
+    long long id = 0;
+    fake::fail_after = 3;
+    EXPECT(gnss_server_submit(s, &c, st.data(), 12, &id) == GNSS_OK);
+    EXPECT(gnss_server_wait(s, id, 10.0) == GNSS_OK);
+    EXPECT(fake::fail_after < 0);
+    long long id2 = 0;
+    EXPECT(gnss_server_submit(s, &c, st.data(), 12, &id2) == GNSS_OK);
+    EXPECT(gnss_server_wait(s, id2, 10.0) == GNSS_OK);
+    EXPECT(fake::recycled_busy == 0);
+    EXPECT(fake::recycled == 0);
+    EXPECT(gnss_server_result(s, id, nullptr, nullptr, nullptr) == GNSS_ERR_CUDA);
+    EXPECT(gnss_server_result(s, id2, nullptr, nullptr, nullptr) == GNSS_OK);
+    // the second one ended well: a third request takes its context over
+    EXPECT(gnss_server_submit(s, &c, st.data(), 12, &id) == GNSS_OK);
+    EXPECT(gnss_server_wait(s, id, 10.0) == GNSS_OK);
+    EXPECT(fake::recycled == 1 && fake::recycled_busy == 0);
+    EXPECT(gnss_server_destroy(s) == GNSS_OK);
+    EXPECT(fake::live == 0);
+    return 0;
+}
+
+int main(int argc, char **argv) {
+    const std::string name = argc > 1 ? argv[1] : "";
+    if (name == "failed_request") return failed_request();
+    return 2;
+}

@@ -34,3 +34,15 @@ def _run(exe: Path, *args: str):
 def test_table_upload_has_arrived_on_return(tmp_path):
     r = _run(_compile(tmp_path / "upload", FAKE / "upload.cpp"))
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.fixture(scope="module")
+def server(tmp_path_factory):
+    return _compile(tmp_path_factory.mktemp("server") / "server", FAKE / "server.cpp", FAKE / "fake_ctx.cpp",
+                    CSRC / "batch.cpp")
+
+
+@pytest.mark.parametrize("scenario", ["failed_request"])
+def test_server(server, scenario):
+    r = _run(server, scenario)
+    assert r.returncode == 0, r.stdout + r.stderr
