@@ -537,7 +537,7 @@ struct gnss_server {
     std::vector<Request *> active;            // scheduler thread only (sizes read under mu)
     std::map<long long, Request *> reqs;      // every request not yet fetched
     std::deque<gnss_ctx *> retired;           // idle contexts of ended requests, for requests of the same geometry (mu)
-    std::vector<gnss_ctx *> spent;            // contexts not offered again, destroyed with the server (mu)
+    std::vector<gnss_ctx *> spent;            // contexts not offered again, destroyed by destroy_spent (mu)
     long long next_id = 1;
     bool stop = false;
     gnss_server_report rep{};
@@ -547,6 +547,25 @@ struct gnss_server {
 
 static double now_s(const gnss_server *s) {
     return std::chrono::duration<double>(Clock::now() - s->t0).count();
+}
+
+// Idle contexts kept for reuse at most (each holds its tables and partial sums, 0.06 - 0.43 MB of device memory);
+// beyond that the one unused for longest is given up.
+constexpr size_t RETIRED_MAX = 64;
+
+// Destroys the contexts given up.  On the thread of a caller who fetches a result, not on the scheduler's: cudaFree
+// synchronises the device.  Every request is fetched after it ended, so none is left when all have been.
+static void destroy_spent(gnss_server *s) {
+    std::vector<gnss_ctx *> spent;
+    {
+        std::lock_guard<std::mutex> lk(s->mu);
+        spent.swap(s->spent);
+    }
+    if (spent.empty()) return;
+    int device = 0;
+    const bool known = cudaGetDevice(&device) == cudaSuccess;
+    for (gnss_ctx *c : spent) gnss_destroy(c);
+    if (known) cudaSetDevice(device);   // the caller's, as it was
 }
 
 // A request that ended well has an idle context (its last event has completed), which may serve another request.  One
@@ -569,16 +588,16 @@ static void req_release_device(gnss_server *s, Request *r) {
         std::lock_guard<std::mutex> lk(s->mu);
         if (idle) s->retired.push_back(r->ctx);
         else s->spent.push_back(r->ctx);
+        while (s->retired.size() > RETIRED_MAX) {
+            s->spent.push_back(s->retired.front());
+            s->retired.pop_front();
+        }
     }
     r->ctx = nullptr;
 }
 
-// Contexts kept for reuse at most; beyond that the one unused for longest is destroyed.
-constexpr size_t RETIRED_MAX = 64;
-
 // A context for a request: one of an ended request of the same geometry, or a new one.
 static gnss_status take_context(gnss_server *s, const gnss_config *cfg, gnss_ctx **out) {
-    gnss_ctx *old = nullptr;
     {
         std::lock_guard<std::mutex> lk(s->mu);
         for (auto it = s->retired.begin(); it != s->retired.end(); ++it)
@@ -587,12 +606,7 @@ static gnss_status take_context(gnss_server *s, const gnss_config *cfg, gnss_ctx
                 s->retired.erase(it);
                 return GNSS_OK;
             }
-        if (s->retired.size() > RETIRED_MAX) {
-            old = s->retired.front();
-            s->retired.pop_front();
-        }
     }
-    if (old) gnss_destroy(old);
     return gnss_create(cfg, out);
 }
 
@@ -909,6 +923,7 @@ gnss_status gnss_server_result(gnss_server *s, long long id, void *host_state_ou
     s->pinned.put(r->h_in);
     s->pinned.put(r->h_out);
     delete r;
+    destroy_spent(s);
     return st;
 }
 

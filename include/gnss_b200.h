@@ -362,7 +362,10 @@ gnss_status gnss_ensemble_autotune(gnss_ensemble *e, int steps, int *choices);
  * the work of requests in flight overlaps on the device.  A finished request
  * keeps its final state and statistics until gnss_server_result.  A
  * request's result is bit-identical to gnss_run_host on the same input,
- * whatever else is in flight.  Times are seconds since the server started. */
+ * whatever else is in flight.  The contexts of ended requests (tables and
+ * partial sums, under 1 MB each, not counted in the budget) are kept for
+ * requests of the same geometry, 64 at most once every ended request has been
+ * fetched.  Times are seconds since the server started. */
 typedef struct gnss_server gnss_server;
 typedef struct gnss_server_config {
     size_t budget_bytes;     /* device memory the server may reserve for requests  */

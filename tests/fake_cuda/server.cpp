@@ -64,8 +64,34 @@ static int failed_request() {
     return 0;
 }
 
+// After a burst of requests (of one geometry, then of several more) has been fetched, no more than 64 idle contexts
+// are left; none was destroyed on the scheduler's thread, and the caller's device is as it was.
+static int idle_contexts() {
+    gnss_server *s = server(4);
+    const int sizes[] = {8, 12, 16};
+    for (int n : sizes) {
+        const gnss_config c = config(n);
+        const std::vector<char> st = state_of(c);
+        std::vector<long long> ids(200);
+        for (long long &id : ids) EXPECT(gnss_server_submit(s, &c, st.data(), 2, &id) == GNSS_OK);
+        EXPECT(cudaSetDevice(1) == cudaSuccess);
+        for (long long id : ids) {
+            EXPECT(gnss_server_wait(s, id, 30.0) == GNSS_OK);
+            EXPECT(gnss_server_result(s, id, nullptr, nullptr, nullptr) == GNSS_OK);
+        }
+        EXPECT(fake::current_device() == 1);
+        EXPECT(fake::live <= 64);
+    }
+    EXPECT(fake::destroyed_elsewhere == 0);
+    EXPECT(fake::recycled_busy == 0);
+    EXPECT(gnss_server_destroy(s) == GNSS_OK);
+    EXPECT(fake::live == 0);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string name = argc > 1 ? argv[1] : "";
     if (name == "failed_request") return failed_request();
+    if (name == "idle_contexts") return idle_contexts();
     return 2;
 }
