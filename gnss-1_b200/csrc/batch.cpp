@@ -602,6 +602,7 @@ static gnss_status take_context(gnss_server *s, const gnss_config *cfg, gnss_ctx
         std::lock_guard<std::mutex> lk(s->mu);
         for (auto it = s->retired.begin(); it != s->retired.end(); ++it)
             if (gnss_recycle(*it, cfg)) {
+                if (cudaSetDevice(cfg->device) != cudaSuccess) return GNSS_ERR_CUDA;   // as gnss_create
                 *out = *it;
                 s->retired.erase(it);
                 return GNSS_OK;

@@ -89,9 +89,31 @@ static int idle_contexts() {
     return 0;
 }
 
+// A submission that takes over an idle context leaves the calling thread on the server's device, as one that creates
+// its context does; its pinned buffers belong there.
+static int device_of_reuse() {
+    const gnss_config c = config(8, 1);
+    const std::vector<char> st = state_of(c);
+    gnss_server *s = server(4, 1);
+    long long a = 0, b = 0;
+    EXPECT(gnss_server_submit(s, &c, st.data(), 2, &a) == GNSS_OK);
+    EXPECT(fake::current_device() == 1 && fake::last_host_alloc_device() == 1);
+    EXPECT(gnss_server_wait(s, a, 10.0) == GNSS_OK);   // not fetched: its pinned buffers are in use
+    EXPECT(cudaSetDevice(0) == cudaSuccess);
+    EXPECT(gnss_server_submit(s, &c, st.data(), 2, &b) == GNSS_OK);
+    EXPECT(fake::recycled == 1);
+    EXPECT(fake::last_host_alloc_device() == 1);
+    EXPECT(fake::current_device() == 1);
+    EXPECT(gnss_server_wait(s, b, 10.0) == GNSS_OK);
+    EXPECT(gnss_server_destroy(s) == GNSS_OK);
+    EXPECT(fake::live == 0);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string name = argc > 1 ? argv[1] : "";
     if (name == "failed_request") return failed_request();
     if (name == "idle_contexts") return idle_contexts();
+    if (name == "device_of_reuse") return device_of_reuse();
     return 2;
 }
