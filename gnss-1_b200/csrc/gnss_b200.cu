@@ -766,16 +766,15 @@ struct SphereCount {
 static SphereCount count_sphere(const gnss_ctx *c) {
     const Geom &g = c->g;
     const int nb = c->elem == sizeof(double2) ? 8 : 16;
-    auto wn = [](int i, int n, double dk) { return (i < n / 2) ? dk * (double)i : dk * ((double)i - (double)n); };
     SphereCount n;
     for (int yc = 0; yc < c->ky_keep.count(); ++yc) {
-        const double k2 = wn(c->ky_keep.expand(yc), g.ny, g.dky);
+        const double k2 = host_wavenum(c->ky_keep.expand(yc), g.ny, g.dky);
         for (int z = 0; z < c->nkz; ++z) {
-            const double k3 = wn(z, g.nz, g.dkz);
+            const double k3 = host_wavenum(z, g.nz, g.dkz);
             int rows = 0;
             for (int xc = 0; xc < c->kx_keep.count(); ++xc) {
-                const double k1 = wn(c->kx_keep.expand(xc), g.nx, g.dkx);
-                rows += (k1 * k1 + k2 * k2) + k3 * k3 > g.kmax2 ? 0 : 1;
+                const double k1 = host_wavenum(c->kx_keep.expand(xc), g.nx, g.dkx);
+                rows += host_ksq(k1, k2, k3) > g.kmax2 ? 0 : 1;
             }
             n.modes += rows;
             n.cols += rows > 0;
@@ -1027,9 +1026,6 @@ static void set_layout(gnss_ctx *c) {
 // which synchronises the device): the error words, the twiddle tables, the
 // FP64 mean-profile line of FP32 contexts (zero: taken from the fields), the
 // tables of the dealiasing sphere for k_passd and the statistics' partial sums.
-// Sphere tables: the kept rows of a column are those whose |index| does not
-// exceed its bound, since k^2 grows with the row's wavenumber; the bounds use
-// the test k^2 > kmax^2 (solver.cu:36) in the reference's order of evaluation.
 // With both pass lengths on k_passd the x passes visit only the tiles (kept
 // ky, column block) whose first column has a mode inside the sphere, and the y
 // passes leave the rows outside it alone; x tiles are 128 bytes wide (8 FP64
@@ -1037,28 +1033,12 @@ static void set_layout(gnss_ctx *c) {
 static gnss_status make_device_block(gnss_ctx *c) {
     const Geom &g = c->g;
     const int nky = c->ky_keep.count(), ncp = c->ncp, nb = c->elem == sizeof(double2) ? 8 : 16;
-    auto wn = [](int i, int n, double dk) { return (i < n / 2) ? dk * (double)i : dk * ((double)i - (double)n); };
-    auto ksq = [](double a, double b, double k) { return (a * a + b * b) + k * k; };
-    std::vector<short> t;
-    std::vector<int> list;
-    if (pd_size(g.nx)) {
-        t.assign((size_t)(nky + 1) * ncp, (short)-1);
-        for (int y = 0; y < nky; ++y) {   // largest kept |kx| of each (ky, kz) column; it falls with kz
-            short *r = t.data() + (size_t)y * ncp;
-            const double ko = wn(c->ky_keep.expand(y), g.ny, g.dky);
-            for (int z = 0, d = g.nx / 2; z < c->nkz; ++z) {
-                while (d >= 0 && ksq(g.dkx * (double)d, ko, wn(z, g.nz, g.dkz)) > g.kmax2) --d;
-                r[z] = (short)d;
-            }
-            for (int b = 0; b < ncp / nb; ++b)
-                if (r[b * nb] >= 0) list.push_back(y << 8 | b);
-        }
-        short *r = t.data() + (size_t)nky * ncp;   // largest kept |ky| of each kz column
-        for (int z = 0, d = g.ny / 2; z < c->nkz; ++z) {
-            while (d >= 0 && ksq(0.0, g.dky * (double)d, wn(z, g.nz, g.dkz)) > g.kmax2) --d;
-            r[z] = (short)d;
-        }
-    }
+    SphereTables sph;
+    if (pd_size(g.nx))
+        sph = sphere_tables({g.nx, g.dkx}, {g.ny, g.dky}, {g.nz, g.dkz}, g.kmax2, nky,
+                            [&](int i) { return c->ky_keep.expand(i); }, c->nkz, ncp, nb);
+    const std::vector<short> &t = sph.bound;
+    const std::vector<int> &list = sph.tiles;
     size_t bytes = 0;
     auto part = [&](size_t n) {   // 256-byte aligned
         const size_t at = bytes;

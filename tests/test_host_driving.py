@@ -9,6 +9,7 @@ import shutil
 import subprocess
 from pathlib import Path
 
+import numpy as np
 import pytest
 
 ROOT = Path(__file__).resolve().parents[1]
@@ -46,3 +47,26 @@ def server(tmp_path_factory):
 def test_server(server, scenario):
     r = _run(server, scenario)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("nx,ny,nz,alias", [(96, 96, 96, 0.75), (64, 128, 48, 15 / 32), (48, 48, 48, 1.0)])
+def test_sphere_tables_do_not_depend_on_fma(tmp_path, nx, ny, nz, alias):
+    """Bounds compiled with contraction to fused multiply-adds allowed equal those of numpy, which rounds every
+    operation, in boxes that put modes like (2 2 1) k exactly on the sphere but for rounding."""
+    fma = ["-mfma"] if " fma " in Path("/proc/cpuinfo").read_text() else []
+    exe = _compile(tmp_path / "sphere", FAKE / "sphere.cpp", flags=["-O3", "-ffp-contract=fast", *fma])
+    for scale in (1.0, 0.31, 0.36, 0.42, 0.44):
+        l = 2 * np.pi * scale
+        r = _run(exe, *(repr(v) for v in (nx, ny, nz, l, l, l, alias)))
+        assert r.returncode == 0, r.stderr
+        bounds, tiles = (np.array(line.split(), dtype=int) for line in r.stdout.splitlines())
+        dk, kmax = 2 * np.pi / l, alias * (nx * np.pi / l)
+        kx = dk * np.arange(nx // 2 + 1)
+        ky = dk * np.where(np.arange(ny) < ny // 2, np.arange(ny), np.arange(ny) - ny)
+        kz = dk * np.array([*range(nz // 2), -nz // 2])
+        inside = ~((kx * kx + (ky * ky)[:, None, None]) + (kz * kz)[:, None] > kmax * kmax)   # [ky][kz][kx]
+        want = inside.sum(axis=2) - 1                                     # the kept |kx| are 0 .. bound
+        y = np.arange(ny // 2 + 1) * dk
+        want_y = (~((y * y) + (kz * kz)[:, None] > kmax * kmax)).sum(axis=1) - 1
+        assert np.array_equal(bounds, np.concatenate([want.ravel(), want_y]))
+        assert np.array_equal(tiles, [i << 8 | k for i in range(ny) for k in range(nz // 2 + 1) if want[i, k] >= 0])
