@@ -18,7 +18,7 @@
 //   axis lies between them) plus a uniform stride.
 //   Measured against the register kernel it replaced (one warp per column, 8
 //   FP64 / 16 FP32 warps per SM), the four passes of a step: 512^3 FP64 with
-//   two scalars 7.98 -> 6.47 ms, 512^3 FP32 4.09 -> 2.95, 256^3 FP32 0.71 ->
+//   two scalars 7.98 -> 6.66 ms, 512^3 FP32 4.09 -> 2.95, 256^3 FP32 0.71 ->
 //   0.36, 192^3 FP32 0.36 -> 0.18 ms.
 //   The dealiasing sphere: rows outside it are not read, tiles outside it are
 //   not visited (21% of the x passes' tiles), and rows no later stage reads
@@ -72,26 +72,12 @@ __device__ __forceinline__ void pd_stage(int t, const CP<typename PkOf<T>::P> *t
             const int k = NS == M ? jj : jj % NS;
 #pragma unroll
             for (int r = 0; r < R; ++r) v[p][r] = ld(jj + r * M);
-            if constexpr (R == 8 && sizeof(T) == 8) {
-                // w^3, w^5, w^6, w^7 as products: three 16-byte reads per lane instead of seven (shared-memory
-                // wavefronts bound the FP64 passes; 512^3, two scalars: 6.66 -> 6.47 ms per step, 192^3 0.326 -> 0.283)
-                using E = CP<typename PkOf<T>::P>;
-                const E w1 = tw[k * TSTEP], w2 = tw[2 * k * TSTEP], w4 = tw[4 * k * TSTEP];
-                const E w3 = cmulp(w1, w2.x, w2.y);
-                auto times = [&](E &x, E w) { x = cmulp(x, w.x, w.y); };
-                times(v[p][1], w1);
-                times(v[p][2], w2);
-                times(v[p][3], w3);
-                times(v[p][4], w4);
-                times(v[p][5], cmulp(w1, w4.x, w4.y));
-                times(v[p][6], cmulp(w2, w4.x, w4.y));
-                times(v[p][7], cmulp(w3, w4.x, w4.y));
-            } else {   // FP32 reads every power: products would add to its rounding error
+            // every power from the table: as products of three of them the FP64 passes took 3% less time (192 points
+            // 13%), and the twiddles' error, 3.3e-17, grew to 7 - 9e-17
 #pragma unroll
-                for (int r = 1; r < R; ++r) {
-                    const CP<typename PkOf<T>::P> w = tw[r * k * TSTEP];
-                    v[p][r] = cmulp(v[p][r], w.x, w.y);
-                }
+            for (int r = 1; r < R; ++r) {
+                const CP<typename PkOf<T>::P> w = tw[r * k * TSTEP];
+                v[p][r] = cmulp(v[p][r], w.x, w.y);
             }
             PDft<R, SIGN>::run(v[p]);
         }
