@@ -25,7 +25,8 @@ template <typename T> using V2 = typename Vec2<T>::type;
 
 template <typename V> __device__ __forceinline__ V cadd(V a, V b) { return V{a.x + b.x, a.y + b.y}; }
 template <typename V> __device__ __forceinline__ V csub(V a, V b) { return V{a.x - b.x, a.y - b.y}; }
-// FP32: real and imaginary part in one packed instruction (sm_100 f32x2)
+// FP32: real and imaginary part in one packed instruction (sm_100 f32x2).  The compiler does not contract these with a
+// product into a fused multiply-add, so where a factor precedes a sum cfma says it.
 template <> __device__ __forceinline__ float2 cadd<float2>(float2 a, float2 b) {
     float2 r;
     asm("{\n\t.reg .b64 p, q, s;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tadd.rn.f32x2 s, p, q;\n\t"
@@ -36,6 +37,17 @@ template <> __device__ __forceinline__ float2 csub<float2>(float2 a, float2 b) {
     float2 r;
     asm("{\n\t.reg .b64 p, q, s;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\tsub.rn.f32x2 s, p, q;\n\t"
         "mov.b64 {%0, %1}, s;\n\t}" : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+// s a + b, rounded once
+template <typename V, typename T> __device__ __forceinline__ V cfma(T s, V a, V b) {
+    return V{fma(s, a.x, b.x), fma(s, a.y, b.y)};
+}
+template <> __device__ __forceinline__ float2 cfma<float2, float>(float s, float2 a, float2 b) {
+    float2 r;
+    asm("{\n\t.reg .b64 p, q, c, d;\n\tmov.b64 p, {%2, %2};\n\tmov.b64 q, {%3, %4};\n\tmov.b64 c, {%5, %6};\n\t"
+        "fma.rn.f32x2 d, p, q, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(s), "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
     return r;
 }
 template <typename V> __device__ __forceinline__ V cmul(V a, V b) {
@@ -100,11 +112,10 @@ template <int S, typename V> struct Dft<3, S, V> {
         const T c3 = T(-0.5);
         const T s3 = T(0.86602540378443864676372317075294);
         V s = cadd(v[1], v[2]), d = csub(v[1], v[2]);
-        V m0 = V{v[0].x + c3 * s.x, v[0].y + c3 * s.y};
-        V jd = mul_si<S>(V{s3 * d.x, s3 * d.y});
+        V m0 = cfma(c3, s, v[0]), jd = mul_si<S>(d);
         v[0] = cadd(v[0], s);
-        v[1] = cadd(m0, jd);
-        v[2] = csub(m0, jd);
+        v[1] = cfma(s3, jd, m0);
+        v[2] = cfma(-s3, jd, m0);
     }
 };
 
@@ -130,17 +141,16 @@ template <int S, typename V> struct Dft<8, S, V> {
         dft4<S>(e0, e1, e2, e3);
         dft4<S>(o0, o1, o2, o3);
         // o1 *= (1 + S i)/sqrt2 ; o2 *= S i ; o3 *= (-1 + S i)/sqrt2
-        V t1 = V{h * (o1.x - T(S) * o1.y), h * (o1.y + T(S) * o1.x)};
+        V t1 = cadd(o1, mul_si<S>(o1)), t3 = csub(mul_si<S>(o3), o3);   // times h below
         V t2 = mul_si<S>(o2);
-        V t3 = V{h * (-o3.x - T(S) * o3.y), h * (-o3.y + T(S) * o3.x)};
         v[0] = cadd(e0, o0);
         v[4] = csub(e0, o0);
-        v[1] = cadd(e1, t1);
-        v[5] = csub(e1, t1);
+        v[1] = cfma(h, t1, e1);
+        v[5] = cfma(-h, t1, e1);
         v[2] = cadd(e2, t2);
         v[6] = csub(e2, t2);
-        v[3] = cadd(e3, t3);
-        v[7] = csub(e3, t3);
+        v[3] = cfma(h, t3, e3);
+        v[7] = cfma(-h, t3, e3);
     }
 };
 

@@ -78,6 +78,7 @@ template <> __device__ __forceinline__ CP<double> cmulp<double>(CP<double> a, do
 }
 
 // ------------------------------------------------------------ small DFTs, natural order
+// Constant factors enter as fused multiply-adds: the packed instructions are not contracted by the compiler.
 template <int S, typename P> __device__ __forceinline__ void pdft4(CP<P> &a0, CP<P> &a1, CP<P> &a2, CP<P> &a3) {
     const CP<P> s02 = a0 + a2, d02 = a0 - a2, s13 = a1 + a3, d13 = a1 - a3;
     a0 = s02 + s13;
@@ -95,13 +96,12 @@ template <int S> struct PDft<2, S> {
 };
 template <int S> struct PDft<3, S> {
     template <typename P> static __device__ __forceinline__ void run(CP<P> *v) {
-        const P c3 = pconst<P>(-0.5), s3 = pconst<P>(0.86602540378443864676372317075294);
+        const P c3 = pconst<P>(-0.5), s3 = pconst<P>(S * 0.86602540378443864676372317075294), n3 = pneg(s3);
         const CP<P> s = v[1] + v[2], d = v[1] - v[2];
         const CP<P> m{pfma(c3, s.x, v[0].x), pfma(c3, s.y, v[0].y)};
-        const CP<P> j{s3 * d.x, s3 * d.y};
         v[0] = v[0] + s;
-        v[1] = add_i<S>(m, j);
-        v[2] = sub_i<S>(m, j);
+        v[1] = {pfma(n3, d.y, m.x), pfma(s3, d.x, m.y)};
+        v[2] = {pfma(s3, d.y, m.x), pfma(n3, d.x, m.y)};
     }
 };
 template <int S> struct PDft<4, S> {
@@ -124,7 +124,7 @@ template <int S> struct PDft<6, S> {   // n = 2 n1 + n2, k = k1 + 3 k2
 };
 template <int S> struct PDft<8, S> {
     template <typename P> static __device__ __forceinline__ void run(CP<P> *v) {
-        const P h = pconst<P>(0.70710678118654752440084436210485);
+        const P h = pconst<P>(0.70710678118654752440084436210485), mh = pneg(h);
         pdft4<S>(v[0], v[2], v[4], v[6]);
         pdft4<S>(v[1], v[3], v[5], v[7]);
         // odd outputs o1, o2, o3 in v[3], v[5], v[7] times W_8^1, W_8^2, W_8^3
@@ -135,11 +135,10 @@ template <int S> struct PDft<8, S> {
         v[4] = e0 - o0;
         v[2] = add_i<S>(e2, o2);
         v[6] = sub_i<S>(e2, o2);
-        const CP<P> t1{h * p1.x, h * p1.y}, t3{h * p3.x, h * p3.y};
-        v[1] = e1 + t1;
-        v[5] = e1 - t1;
-        v[3] = e3 - t3;
-        v[7] = e3 + t3;
+        v[1] = {pfma(h, p1.x, e1.x), pfma(h, p1.y, e1.y)};
+        v[5] = {pfma(mh, p1.x, e1.x), pfma(mh, p1.y, e1.y)};
+        v[3] = {pfma(mh, p3.x, e3.x), pfma(mh, p3.y, e3.y)};
+        v[7] = {pfma(h, p3.x, e3.x), pfma(h, p3.y, e3.y)};
     }
 };
 

@@ -5,7 +5,8 @@ and inverse, against 80-bit transforms on the host.  The bound is the error
 that the table-driven radix-8 passes have on the same fields (relative RMS, 48
 fields each, below), and 1% more: the two radix plans of a length differ by
 less than that, and the sampling error of an RMS over 48 fields is 0.3%.
-Twiddles formed as products of table entries raise it by 2 to 10%.
+Twiddles formed as products of table entries raise it by 2 to 10%, a factor
+and a sum rounded apart in the small transforms by 1 to 4%.
 """
 import numpy as np
 import pytest
@@ -21,6 +22,13 @@ BOUND = {
     (0, 1): {48: (2.030e-16, 1.988e-16), 64: (2.098e-16, 1.998e-16), 96: (2.103e-16, 2.080e-16),
              128: (2.241e-16, 2.129e-16), 192: (2.243e-16, 2.161e-16), 256: (2.396e-16, 2.271e-16),
              384: (2.372e-16, 2.260e-16), 512: (2.508e-16, 2.355e-16)},
+    (1, 0): {48: (1.099e-07, 1.072e-07), 64: (1.074e-07, 1.076e-07), 96: (1.190e-07, 1.135e-07),
+             128: (1.167e-07, 1.177e-07), 192: (1.269e-07, 1.202e-07), 256: (1.193e-07, 1.188e-07),
+             384: (1.262e-07, 1.215e-07), 512: (1.283e-07, 1.268e-07)},
+    (1, 1): {48: (1.097e-07, 1.080e-07), 64: (1.071e-07, 1.082e-07), 96: (1.195e-07, 1.145e-07),
+             128: (1.169e-07, 1.177e-07), 192: (1.274e-07, 1.207e-07), 256: (1.193e-07, 1.195e-07),
+             384: (1.263e-07, 1.224e-07), 512: (1.284e-07, 1.274e-07)},
+    (1, 2): {48: (1.125e-07, 1.102e-07), 384: (1.294e-07, 1.262e-07)},
 }
 # radix 6 rounds by its own pattern: forward 1% under, inverse 2.6% over the bound of 8 2 3
 SKIP = {(0, 0, 48), (0, 1, 48)}
