@@ -107,18 +107,15 @@ template <int S> struct PDft<3, S> {
 template <int S> struct PDft<4, S> {
     template <typename P> static __device__ __forceinline__ void run(CP<P> *v) { pdft4<S>(v[0], v[1], v[2], v[3]); }
 };
-template <int S> struct PDft<6, S> {   // n = 2 n1 + n2, k = k1 + 3 k2
+template <int S> struct PDft<6, S> {   // n = 3 n1 + 2 n2, k = 3 k1 + 4 k2 (mod 6): no twiddles
     template <typename P> static __device__ __forceinline__ void run(CP<P> *v) {
-        const P h = pconst<P>(0.5), mh = pconst<P>(-0.5), s3 = pconst<P>(S * 0.86602540378443864676372317075294);
-        CP<P> a[3] = {v[0], v[2], v[4]}, b[3] = {v[1], v[3], v[5]};
+        CP<P> a[3] = {v[0], v[2], v[4]}, b[3] = {v[3], v[5], v[1]};
         PDft<3, S>::run(a);
         PDft<3, S>::run(b);
-        b[1] = cmulp(b[1], h, s3);
-        b[2] = cmulp(b[2], mh, s3);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            v[k] = a[k] + b[k];
-            v[k + 3] = a[k] - b[k];
+        for (int k2 = 0; k2 < 3; ++k2) {
+            v[(4 * k2) % 6] = a[k2] + b[k2];
+            v[(3 + 4 * k2) % 6] = a[k2] - b[k2];
         }
     }
 };

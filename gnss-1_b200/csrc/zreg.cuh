@@ -126,22 +126,17 @@ template <typename T, int N> struct ZRCfg {
     }
 };
 
-// 6-point DFT in natural order: n = 2 n1 + n2, k = k1 + 3 k2 (two 3-point
-// DFTs, twiddles W_6^(n2 k1), one 2-point stage).
+// 6-point DFT in natural order: n = 3 n1 + 2 n2, k = 3 k1 + 4 k2 (mod 6), two
+// 3-point DFTs and one 2-point stage without twiddles.
 template <int S, typename V> struct Dft<6, S, V> {
     static __device__ __forceinline__ void run(V *v) {
-        using T = decltype(v[0].x);
-        const T h = T(0.5);
-        const T s3 = T(S) * T(0.86602540378443864676372317075294);
-        V a[3] = {v[0], v[2], v[4]}, b[3] = {v[1], v[3], v[5]};
+        V a[3] = {v[0], v[2], v[4]}, b[3] = {v[3], v[5], v[1]};
         Dft<3, S, V>::run(a);
         Dft<3, S, V>::run(b);
-        b[1] = V{h * b[1].x - s3 * b[1].y, h * b[1].y + s3 * b[1].x};     // W_6^1 = 1/2 + i S sqrt(3)/2
-        b[2] = V{-h * b[2].x - s3 * b[2].y, -h * b[2].y + s3 * b[2].x};   // W_6^2 = -1/2 + i S sqrt(3)/2
 #pragma unroll
-        for (int k1 = 0; k1 < 3; ++k1) {
-            v[k1] = cadd(a[k1], b[k1]);
-            v[k1 + 3] = csub(a[k1], b[k1]);
+        for (int k2 = 0; k2 < 3; ++k2) {
+            v[(4 * k2) % 6] = cadd(a[k2], b[k2]);
+            v[(3 + 4 * k2) % 6] = csub(a[k2], b[k2]);
         }
     }
 };
