@@ -107,11 +107,11 @@ template <typename T, int N> struct PassLaunch {
     }
     static cudaError_t zpass(int dir, const FieldSet<T> &f, int nfields, long long nlines, int nz2, T scale,
                              const void *tw, cudaStream_t s) {
-        // register transforms at every length they serve (192 x 256 x 128 FP64, forward + inverse with all passes:
-        // 241 us with k_zpass, 202 with k_zline)
-        if constexpr (zr_size(N)) {
+        // register transforms where they round no more than k_zpass; forward + inverse with all passes:
+        // 192 x 256 x 128 FP64 241 us with k_zpass, 202 with k_zline; FP32 123 and 113 us, 256 x 256 x 512 689 and 526
+        if constexpr (zline_size(N, sizeof(T) == 8)) {
             using Z = ZRCfg<T, N>;
-            const int smem = (Z::LOGE * 32 + ZLINE_WARPS * Z::SCR) * (int)sizeof(V2<T>);
+            const int smem = (Z::FINE_ROWS * 32 + ZLINE_WARPS * Z::SCR) * (int)sizeof(V2<T>);
             auto kern = dir < 0 ? k_zline<T, N, -1> : k_zline<T, N, +1>;
             cudaError_t e = prep_smem(kern, smem);
             if (e != cudaSuccess) return e;

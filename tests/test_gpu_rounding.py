@@ -29,7 +29,12 @@ BOUND = {
     (1, 1): {48: (1.097e-07, 1.080e-07), 64: (1.071e-07, 1.082e-07), 96: (1.195e-07, 1.145e-07),
              128: (1.169e-07, 1.177e-07), 192: (1.274e-07, 1.207e-07), 256: (1.193e-07, 1.195e-07),
              384: (1.263e-07, 1.224e-07), 512: (1.284e-07, 1.274e-07)},
-    (1, 2): {48: (1.125e-07, 1.102e-07), 384: (1.294e-07, 1.262e-07)},
+    (0, 2): {48: (2.089e-16, 2.039e-16), 64: (2.162e-16, 2.084e-16), 96: (2.165e-16, 2.146e-16),
+             128: (2.297e-16, 2.221e-16), 192: (2.304e-16, 2.243e-16), 256: (2.378e-16, 2.299e-16),
+             384: (2.434e-16, 2.353e-16), 512: (2.535e-16, 2.460e-16)},
+    (1, 2): {48: (1.125e-07, 1.102e-07), 64: (1.099e-07, 1.105e-07), 96: (1.192e-07, 1.156e-07),
+             128: (1.163e-07, 1.168e-07), 192: (1.236e-07, 1.210e-07), 256: (1.216e-07, 1.218e-07),
+             384: (1.294e-07, 1.262e-07), 512: (1.271e-07, 1.269e-07)},
 }
 
 
