@@ -102,9 +102,12 @@ template <typename T, int N> struct ZRCfg {
     static constexpr bool SHFL = E != 8 && E != 16;     // lane-shuffle scheme (no transpose)
     static constexpr int G = SHFL ? 1 : 32 / E;         // lanes per group in step B (transpose scheme)
     static constexpr int S = 32 + G;                    // transpose row stride (conflict-free both ways)
-    // table rows: the powers W_N^(lane 2^b), b < LOGE, of the transpose scheme's step-A twiddles; the shuffle scheme
-    // reads W_N^(lane k1), k1 = 1 .. E-1, then W_32^lane
-    static constexpr int LOGE = SHFL ? E : (E == 16 ? 4 : 3);
+    // table rows: the powers W_N^(lane r), r = 1 2 3 4 (and 8 12 where E = 16), of the transpose scheme's step-A
+    // twiddles, so that each other one is a product of two; FP64 lines of 512 points keep to r = 1 2 4 8 (POW2), since
+    // their staged lines fill the shared memory (two scalars, 192 kept kz columns).  The shuffle scheme reads
+    // W_N^(lane k1), k1 = 1 .. E-1, then W_32^lane.
+    static constexpr bool POW2 = E == 16 && sizeof(T) == 8;
+    static constexpr int ROWS = SHFL ? E : POW2 ? 4 : (E == 16 ? 6 : 4);
     // line padding.  Transpose scheme: a warp's stores of a transform's
     // output (zr_out_index: lane groups j = lane % G at E^2 sigma(j) apart,
     // lanes of a group on consecutive entries) take one wavefront per 128
@@ -126,7 +129,8 @@ template <typename T, int N> struct ZRCfg {
     // index into the length-N table exp(-2 pi i j / N) of twiddle-table entry i
     __host__ __device__ static constexpr int tw_index(int i) {
         const int row = i >> 5, l = i & 31;
-        return SHFL ? (row < E - 1 ? (l * (row + 1)) % N : (E * l) % N) : (l << row) % N;
+        if (SHFL) return row < E - 1 ? (l * (row + 1)) % N : (E * l) % N;
+        return (l * (POW2 ? 1 << row : row < 4 ? row + 1 : 4 * row - 8)) % N;
     }
     // the table of k_zline: every power W_N^(lane k1), k1 = 1 .. E-1 (and W_32^lane)
     static constexpr int FINE_ROWS = SHFL ? E : E - 1;
@@ -276,7 +280,9 @@ __device__ __forceinline__ void zs_fft(int lane, V2<T> *x, const V2<T> *tws) {
 }
 
 // x[k1] *= W_N^(SIGN lane k1), the step-A twiddles of zr_fft (transpose scheme): FINE reads every power from the table
-// of k_zline, else the others are products of the powers 2^b.
+// of k_zline, else those outside the table are products of entries.  (With rows for the powers of two only, powers like
+// 7 and 13 take two products: a step's FP32 right-hand side was 2% and 5% further off at 256 and 512 points, in the
+// same time.)
 template <typename T, int N, int SIGN, bool FINE>
 __device__ __forceinline__ void zr_twiddle(int lane, V2<T> *x, const V2<T> *tws) {
     using V = V2<T>;
@@ -290,18 +296,18 @@ __device__ __forceinline__ void zr_twiddle(int lane, V2<T> *x, const V2<T> *tws)
 #pragma unroll
         for (int r = 1; r < E; ++r) x[r] = cmul(x[r], tw_at(r - 1));
     } else {
-        const V w1 = tw_at(0), w2 = tw_at(1), w4 = tw_at(2);
-        const V w3 = cmul(w1, w2);
+        constexpr bool POW2 = ZRCfg<T, N>::POW2;
+        const V w1 = tw_at(0), w2 = tw_at(1), w3 = POW2 ? cmul(w1, w2) : tw_at(2), w4 = tw_at(POW2 ? 2 : 3);
         if constexpr (E == 16) {
-            const V w8 = tw_at(3);
+            const V w8 = tw_at(POW2 ? 3 : 4), w12 = POW2 ? cmul(w4, w8) : tw_at(5);
             x[8] = cmul(x[8], w8);
             x[9] = cmul(x[9], cmul(w1, w8));
             x[10] = cmul(x[10], cmul(w2, w8));
             x[11] = cmul(x[11], cmul(w3, w8));
-            x[12] = cmul(x[12], cmul(w4, w8));
-            x[13] = cmul(x[13], cmul(cmul(w1, w4), w8));
-            x[14] = cmul(x[14], cmul(cmul(w2, w4), w8));
-            x[15] = cmul(x[15], cmul(cmul(w3, w4), w8));
+            x[12] = cmul(x[12], w12);
+            x[13] = cmul(x[13], cmul(w1, w12));
+            x[14] = cmul(x[14], cmul(w2, w12));
+            x[15] = cmul(x[15], cmul(w3, w12));
         }
         x[1] = cmul(x[1], w1);
         x[2] = cmul(x[2], w2);
@@ -714,7 +720,7 @@ template <typename T, int N, int NPH> struct ZPipe {   // FP32
     // blocks per SM the registers are sized for
     static constexpr int MINB = NPH <= 9 ? (N <= 192 ? 3 : 2) : NPH == 12 || N <= 192 ? 2 : 1;
     __host__ __device__ static constexpr int smem_bytes(int nraw, int ncp) {
-        return (Z::LOGE * 32 + NPH * LINE + NOUT * FSCR + nraw * 2 * ncp) * (int)sizeof(V2<T>) + 16 + ncp * (int)sizeof(T);
+        return (Z::ROWS * 32 + NPH * LINE + NOUT * FSCR + nraw * 2 * ncp) * (int)sizeof(V2<T>) + 16 + ncp * (int)sizeof(T);
     }
 };
 
@@ -754,7 +760,7 @@ k_zpipe(const __grid_constant__ FieldSet<T> f, const __grid_constant__ ZRecipeSe
     const unsigned raw_bytes = (unsigned)(rawf * sizeof(V));
     extern __shared__ __align__(16) unsigned char smem_raw[];
     V *tws = reinterpret_cast<V *>(smem_raw);
-    V *lines = tws + Z::LOGE * 32;
+    V *lines = tws + Z::ROWS * 32;
     V *fscr = lines + NPH * C::LINE;
     V *raw = fscr + C::NOUT * C::FSCR;
     uint64_t *bar = reinterpret_cast<uint64_t *>(raw + NRAW * rawf);
@@ -762,7 +768,7 @@ k_zpipe(const __grid_constant__ FieldSet<T> f, const __grid_constant__ ZRecipeSe
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     long long next = blockIdx.x;
     if (next >= npairs) return;   // uniform for the block
-    for (int i = threadIdx.x; i < Z::LOGE * 32; i += C::NT) tws[i] = tw[Z::tw_index(i)];
+    for (int i = threadIdx.x; i < Z::ROWS * 32; i += C::NT) tws[i] = tw[Z::tw_index(i)];
     for (int k = threadIdx.x; k < ncp; k += C::NT) tkz[k] = (T)wavenum(k, N, dkz);
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
@@ -902,7 +908,7 @@ template <typename T, int N, int NPH> struct ZWs {
     // blocks per SM the registers are sized for
     static constexpr int MINB = N == 512 ? 1 : N == 256 ? (NPH == 9 ? 2 : 1) : (NPH <= 12 ? 2 : 1);
     __host__ __device__ static constexpr int smem_bytes(int nraw, int ncp) {
-        return (Z::LOGE * 32 + (NPH + NOUT) * Z::SCR + nraw * 2 * ncp) * (int)sizeof(V2<T>) + 16 + ncp * (int)sizeof(T);
+        return (Z::ROWS * 32 + (NPH + NOUT) * Z::SCR + nraw * 2 * ncp) * (int)sizeof(V2<T>) + 16 + ncp * (int)sizeof(T);
     }
 };
 
@@ -935,7 +941,7 @@ k_zws(const __grid_constant__ FieldSet<T> f, const __grid_constant__ ZRecipeSet 
     const unsigned raw_bytes = (unsigned)(rawf * sizeof(V));
     extern __shared__ __align__(16) unsigned char smem_raw[];
     V *tws = reinterpret_cast<V *>(smem_raw);
-    V *lines = tws + Z::LOGE * 32;   // NPH + NOUT lines, one per warp
+    V *lines = tws + Z::ROWS * 32;   // NPH + NOUT lines, one per warp
     V *raw = lines + (NPH + C::NOUT) * SCR;
     uint64_t *bar = reinterpret_cast<uint64_t *>(raw + (STAGED ? NRAW * rawf : 0));
     T *tkz = reinterpret_cast<T *>(bar + 2);   // kz wavenumbers of the kept modes (ncp entries)
@@ -943,7 +949,7 @@ k_zws(const __grid_constant__ FieldSet<T> f, const __grid_constant__ ZRecipeSet 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     long long pair = blockIdx.x;
     if (pair >= npairs) return;   // uniform for the block
-    for (int i = threadIdx.x; i < Z::LOGE * 32; i += C::NT) tws[i] = tw[Z::tw_index(i)];
+    for (int i = threadIdx.x; i < Z::ROWS * 32; i += C::NT) tws[i] = tw[Z::tw_index(i)];
     for (int k = threadIdx.x; k < ncp; k += C::NT) tkz[k] = (T)wavenum(k, N, dkz);
     if (threadIdx.x == 0) {
         stop = 0;

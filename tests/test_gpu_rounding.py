@@ -70,3 +70,57 @@ def test_transform_rounding(torch_cuda, precision, axis, n):
         got = np.array(got)
         err = float(np.sqrt((np.abs(got - want) ** 2).sum() / (np.abs(want) ** 2).sum()))
         assert err <= 1.01 * bound
+
+
+# right-hand side (u, v, w, s) of a step on such fields with every transform's twiddles exact or one product away
+STEP_BOUND = {
+    (64, 64, 64, 0): (4.443e-16, 4.487e-16, 4.367e-16, 3.895e-16),
+    (64, 64, 512, 0): (4.562e-16, 4.526e-16, 4.454e-16, 3.947e-16),
+    (64, 64, 256, 1): (2.628e-07, 2.645e-07, 2.565e-07, 2.464e-07),
+    (64, 64, 512, 1): (2.882e-07, 2.859e-07, 2.850e-07, 2.707e-07),
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,nz,precision", list(STEP_BOUND))
+def test_step_rounding(torch_cuda, nx, ny, nz, precision):
+    """The history after an Euler step (the projected nonlinear term) against 80-bit floats."""
+    import scipy.fft
+    import gnss_b200 as G
+    torch = torch_cuda
+    cplx = np.complex128 if precision == 0 else np.complex64
+    rng = np.random.default_rng(nx * 1000003 + ny * 1009 + nz)
+    kx = np.fft.fftfreq(nx, 1 / nx)[None, :, None]
+    ky = np.fft.fftfreq(ny, 1 / ny)[:, None, None]
+    kz = np.arange(nz // 2 + 1.0)[None, None, :]
+    k2 = kx * kx + ky * ky + kz * kz
+    keep = k2 <= (2 / 3 * nx / 2) ** 2
+    st = [np.where(keep, np.fft.rfftn(rng.standard_normal((nx, ny, nz))).transpose(1, 0, 2) * (1 + k2 / 64) ** -1.4,
+                   0).astype(cplx) for _ in range(4)]
+    with G.Context(nx=nx, ny=ny, nz=nz, precision=precision, re=500.0, dt=1e-3) as ctx:
+        dev = [torch.from_numpy(np.ascontiguousarray(f)).cuda() for f in st]
+        hist = [torch.zeros_like(t) for t in dev]
+        ctx.solver_ps(dev, hist, euler=True)
+        got = [to_host(t) for t in hist]
+
+    def phys(f):
+        t = scipy.fft.ifftn(f.transpose(1, 0, 2), axes=(0, 1))
+        t[..., 0].imag = 0
+        t[..., -1].imag = 0
+        return scipy.fft.irfft(t, n=nz, axis=2)
+
+    def spec(p):
+        return scipy.fft.rfftn(p).transpose(1, 0, 2)
+
+    u, v, w, s = (f.astype(np.clongdouble) for f in st)
+    up, vp, wp = phys(u), phys(v), phys(w)
+    o1, o2, o3 = (phys(1j * t) for t in (ky * w - kz * v, kz * u - kx * w, kx * v - ky * u))
+    n = [spec(o2 * wp - o3 * vp), spec(o3 * up - o1 * wp), spec(o1 * vp - o2 * up)]
+    pr = (kx * n[0] + ky * n[1] + kz * n[2]) / np.maximum(k2, 1).astype(np.longdouble)
+    want = [k * pr - f for k, f in zip((kx, ky, kz), n)]
+    want.append(-spec(up * phys(1j * kx * s) + vp * phys(1j * ky * s) + wp * phys(1j * kz * s)))
+    for g, x, bound in zip(got, want, STEP_BOUND[nx, ny, nz, precision]):
+        x = np.where(keep, x, 0)
+        x[0, 0, 0] = 0
+        err = float(np.sqrt((np.abs(g - x) ** 2).sum() / (np.abs(x) ** 2).sum()))
+        assert err <= 1.01 * bound
