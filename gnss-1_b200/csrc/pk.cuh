@@ -96,7 +96,8 @@ template <int S> struct PDft<2, S> {
 };
 template <int S> struct PDft<3, S> {
     template <typename P> static __device__ __forceinline__ void run(CP<P> *v) {
-        const P c3 = pconst<P>(-0.5), s3 = pconst<P>(S * 0.86602540378443864676372317075294), n3 = pneg(s3);
+        const P c3 = pconst<P>(-0.5), s3 = pconst<P>(S * 0.86602540378443864676372317075294);
+        const P n3 = pconst<P>(-S * 0.86602540378443864676372317075294);
         const CP<P> s = v[1] + v[2], d = v[1] - v[2];
         const CP<P> m{pfma(c3, s.x, v[0].x), pfma(c3, s.y, v[0].y)};
         v[0] = v[0] + s;
@@ -121,7 +122,7 @@ template <int S> struct PDft<6, S> {   // n = 3 n1 + 2 n2, k = 3 k1 + 4 k2 (mod 
 };
 template <int S> struct PDft<8, S> {
     template <typename P> static __device__ __forceinline__ void run(CP<P> *v) {
-        const P h = pconst<P>(0.70710678118654752440084436210485), mh = pneg(h);
+        const P h = pconst<P>(0.70710678118654752440084436210485), mh = pconst<P>(-0.70710678118654752440084436210485);
         pdft4<S>(v[0], v[2], v[4], v[6]);
         pdft4<S>(v[1], v[3], v[5], v[7]);
         // odd outputs o1, o2, o3 in v[3], v[5], v[7] times W_8^1, W_8^2, W_8^3
