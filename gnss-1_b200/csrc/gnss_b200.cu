@@ -757,42 +757,14 @@ gnss_status gnss_check(gnss_ctx *c, void *stream) {
     return GNSS_OK;
 }
 
-// What of the kept box lies inside the dealiasing sphere: modes (the ones k_update touches after the first step);
-// columns (ky, kz) with a kept mode, and those of the x passes' tiles; modes the x forward pass stores (all columns of
-// a tile with the rows of its first one).
-struct SphereCount {
-    double modes = 0, cols = 0, tile_cols = 0, stored = 0;
-};
-static SphereCount count_sphere(const gnss_ctx *c) {
-    const Geom &g = c->g;
-    const int nb = c->elem == sizeof(double2) ? 8 : 16;
-    SphereCount n;
-    for (int yc = 0; yc < c->ky_keep.count(); ++yc) {
-        const double k2 = host_wavenum(c->ky_keep.expand(yc), g.ny, g.dky);
-        for (int z = 0; z < c->nkz; ++z) {
-            const double k3 = host_wavenum(z, g.nz, g.dkz);
-            int rows = 0;
-            for (int xc = 0; xc < c->kx_keep.count(); ++xc) {
-                const double k1 = host_wavenum(c->kx_keep.expand(xc), g.nx, g.dkx);
-                rows += host_ksq(k1, k2, k3) > g.kmax2 ? 0 : 1;
-            }
-            n.modes += rows;
-            n.cols += rows > 0;
-            if (z % nb == 0 && rows > 0) {
-                n.tile_cols += nb;
-                n.stored += (double)nb * rows;
-            }
-        }
-    }
-    return n;
-}
-
 gnss_status gnss_stage_bytes(const gnss_ctx *c, double *bytes) {
     if (!c || !bytes) return GNSS_ERR_INVALID;
     const double e = (double)c->elem;
     const int nf = 3 + c->cfg.n_scalars;
     const double nkx = c->kx_keep.count(), nky = c->ky_keep.count();
-    const SphereCount n = count_sphere(c);
+    const SphereCount n = count_sphere({c->g.nx, c->g.dkx}, {c->g.ny, c->g.dky}, {c->g.nz, c->g.dkz}, c->g.kmax2,
+                                       c->ky_keep.count(), [&](int i) { return c->ky_keep.expand(i); }, c->nkz,
+                                       c->elem == sizeof(double2) ? 8 : 16);
     // the x / y intermediates hold what lies in the sphere (both passes on k_passd), or the whole kept box
     const bool sphere = c->xlist && (c->pvariant == GNSS_VARIANT_AUTO || c->pvariant == GNSS_VARIANT_REGISTER);
     const double pw = sphere ? (double)c->g.nx * n.tile_cols : (double)c->p_elems;   // P as its tiles are stored

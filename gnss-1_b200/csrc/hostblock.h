@@ -65,4 +65,30 @@ inline cudaError_t upload_and_wait(void *dst, const void *src, size_t bytes) {
     return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
 }
 
+// What of the kept box lies inside the sphere: modes (the ones k_update touches after the first step); columns (ky, kz)
+// with a kept mode, and those of the x passes' tiles; modes the x forward pass stores (all columns of a tile with the
+// rows of its first one).  From the columns' bounds, a few operations each: the box has millions of modes.
+struct SphereCount {
+    double modes = 0, cols = 0, tile_cols = 0, stored = 0;
+};
+template <class Ky>
+SphereCount count_sphere(SphereAxis x, SphereAxis y, SphereAxis z, double kmax2, int nky, Ky ky, int nkz, int nb) {
+    SphereCount n;
+    for (int i = 0; i < nky; ++i) {
+        const double ko = host_wavenum(ky(i), y.n, y.dk);
+        for (int k = 0, d = x.n / 2; k < nkz; ++k) {
+            while (d >= 0 && host_ksq(x.dk * (double)d, ko, host_wavenum(k, z.n, z.dk)) > kmax2) --d;
+            if (d < 0) break;   // the bounds fall with kz
+            const int rows = 2 * d >= x.n ? x.n : 2 * d + 1;
+            n.modes += rows;
+            n.cols += 1;
+            if (k % nb == 0) {
+                n.tile_cols += nb;
+                n.stored += (double)nb * rows;
+            }
+        }
+    }
+    return n;
+}
+
 }  // namespace gnss

@@ -1,4 +1,4 @@
-// Prints the bounds of sphere_tables for the grid and box in the arguments:
+// Prints the bounds of sphere_tables and the counts of count_sphere (8 columns per tile) for the grid and box in the arguments:
 // nx ny nz lx ly lz alias_filter.
 #include <cmath>
 #include <cstdio>
@@ -18,5 +18,9 @@ int main(int, char **argv) {
     std::printf("\n");
     for (int e : t.tiles) std::printf("%d ", e);
     std::printf("\n");
+    const gnss::SphereCount n =
+        gnss::count_sphere({nx, 2 * M_PI / lx}, {ny, 2 * M_PI / ly}, {nz, 2 * M_PI / lz}, kmax * kmax, ny,
+                           [](int i) { return i; }, nkz, 8);
+    std::printf("%.0f %.0f %.0f %.0f\n", n.modes, n.cols, n.tile_cols, n.stored);
     return 0;
 }

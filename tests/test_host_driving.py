@@ -59,7 +59,7 @@ def test_sphere_tables_do_not_depend_on_fma(tmp_path, nx, ny, nz, alias):
         l = 2 * np.pi * scale
         r = _run(exe, *(repr(v) for v in (nx, ny, nz, l, l, l, alias)))
         assert r.returncode == 0, r.stderr
-        bounds, tiles = (np.array(line.split(), dtype=int) for line in r.stdout.splitlines())
+        bounds, tiles, counts = (np.array(line.split(), dtype=int) for line in r.stdout.splitlines())
         dk, kmax = 2 * np.pi / l, alias * (nx * np.pi / l)
         kx = dk * np.arange(nx // 2 + 1)
         ky = dk * np.where(np.arange(ny) < ny // 2, np.arange(ny), np.arange(ny) - ny)
@@ -69,4 +69,8 @@ def test_sphere_tables_do_not_depend_on_fma(tmp_path, nx, ny, nz, alias):
         y = np.arange(ny // 2 + 1) * dk
         want_y = (~((y * y) + (kz * kz)[:, None] > kmax * kmax)).sum(axis=1) - 1
         assert np.array_equal(bounds, np.concatenate([want.ravel(), want_y]))
+        rows = np.where(2 * want >= nx, nx, 2 * want + 1)   # modes +-kx of a column
+        first = rows[:, ::8]
+        assert list(counts) == [rows[want >= 0].sum(), (want >= 0).sum(), 8 * (first > 0).sum(),
+                                8 * first[first > 0].sum()]
         assert np.array_equal(tiles, [i << 8 | k for i in range(ny) for k in range(nz // 2 + 1) if want[i, k] >= 0])
