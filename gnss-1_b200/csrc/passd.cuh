@@ -70,14 +70,25 @@ __device__ __forceinline__ void pd_stage(int t, const CP<typename PkOf<T>::P> *t
         const int jj = t + p * TPC;
         if (M % TPC == 0 || jj < M) {
             const int k = NS == M ? jj : jj % NS;
-#pragma unroll
-            for (int r = 0; r < R; ++r) v[p][r] = ld(jj + r * M);
-            // every power from the table: as products of three of them the FP64 passes took 3% less time (192 points
-            // 13%), and the twiddles' error, 3.3e-17, grew to 7 - 9e-17
+            // Every power from the table: as products of three of them the twiddles' error, 3.3e-17, grew to 7 - 9e-17.
+            // Each load stands beside its product, else seven twiddles in flight spill (FP64 passes of 384 x 384 x 256:
+            // 2.71 ms, 2.19 so); where the powers' addresses, kept from tile to tile, spill too (FP64 192) or make
+            // the loads wait (512), they are formed on the way (192^3 319 -> 288 us; 512 x 512 x 256 with two scalars
+            // 5.67 -> 5.45 ms; at 384 this spills instead).
+            constexpr bool CHAIN = N == 512 || (N == 192 && sizeof(T) == 8);
+            const CP<typename PkOf<T>::P> *wr = tw;
+            int step = k * TSTEP;
+            v[p][0] = ld(jj);
 #pragma unroll
             for (int r = 1; r < R; ++r) {
-                const CP<typename PkOf<T>::P> w = tw[r * k * TSTEP];
-                v[p][r] = cmulp(v[p][r], w.x, w.y);
+                if constexpr (CHAIN) {
+                    asm volatile("" : "+r"(step));
+                    wr += step;
+                } else {
+                    wr = tw + r * k * TSTEP;
+                }
+                const CP<typename PkOf<T>::P> w = *wr;
+                v[p][r] = cmulp(ld(jj + r * M), w.x, w.y);
             }
             PDft<R, SIGN>::run(v[p]);
         }
