@@ -48,7 +48,9 @@ template <typename T, int N> struct PDCfg {
     static constexpr int NT = U * TPC;
     static constexpr int BUFS = 2;
     static constexpr int SMEM = BUFS * N * U * 16 + N * 16 + N * 8;   // tiles, twiddles, row wavenumbers
-    static constexpr int THREADS = 768;   // threads per SM the registers are sized for (80 each)
+    // threads per SM the registers are sized for: 80 each, and 96 where 80 spill and few tiles make up for it (48^3
+    // FP32 transform 16.5 -> 14.5 us, FP64 step 41.5 -> 37.3; 64^3 FP64 step 41.1 -> 38.7; 64 x 512 x 512 unchanged)
+    static constexpr int THREADS = N == 48 || (N == 64 && W == 1) ? 640 : 768;
     static constexpr int FIT = (227 * 1024) / (SMEM + 1024);
     static constexpr int MINB = FIT < THREADS / NT ? FIT : THREADS / NT;
     static constexpr int RL = pd_radix(N, pd_stages(N) - 1);   // radix of the last stage
