@@ -56,12 +56,11 @@ __host__ __device__ constexpr bool pd_size(int n) {
 // (input field, tile) with a tile of NB columns x N rows, rows of 128 bytes.
 // Every input tile is read from HBM once and may produce up to two outputs,
 // each the transform of the tile times a spectral multiplier:
-//   V_ONE 1, V_IK_ROW i k_row, V_IK_OUT i k_outer, V_IK_COL i k_col,
-//   V_LAP -(k_row^2 + k_outer^2 + k_col^2),
+//   V_ONE 1, V_IK_ROW i k_row, V_LAP -(k_row^2 + k_outer^2 + k_col^2),
 // optionally after the dealias mask k^2 > kmax^2 -> 0 (all three wavenumbers
 // are known in the first, spectral-side pass).  Outputs are written with
 // their own strides (a transposed store for the x passes).
-enum : signed char { V_ONE = 0, V_IK_ROW = 1, V_IK_OUT = 2, V_IK_COL = 3, V_LAP = 4 };
+enum : signed char { V_ONE = 0, V_IK_ROW = 1, V_LAP = 2 };
 
 // |row index| of a transform row (the Nyquist row counts as N/2)
 template <int N> __device__ __forceinline__ int row_dist(int r) { return r <= N / 2 ? r : N - r; }
@@ -223,8 +222,6 @@ k_pass(const __grid_constant__ PassPtrs<T> P, const __grid_constant__ PassSpec s
                 if (sp.mask && k2 > sp.kmax2) return V{T(0), T(0)};   // dealias mask (solver.cu:36)
                 switch (mul) {
                     case V_IK_ROW: return V{(T)(-kr) * a.y, (T)kr * a.x};
-                    case V_IK_OUT: return V{(T)(-k_out) * a.y, (T)k_out * a.x};
-                    case V_IK_COL: return V{(T)(-kc) * a.y, (T)kc * a.x};
                     case V_LAP: return V{(T)(-k2) * a.x, (T)(-k2) * a.y};
                     default: return a;
                 }

@@ -41,8 +41,9 @@ template <typename T, int N> struct PassLaunch {
     static bool rows16(long long row, long long outer, long long member) {
         return sizeof(T) == 8 || ((row | outer | member) & 1) == 0;
     }
-    // Members of a batch (sp.nmem > 1) run the MB instantiations, which exist for the register lengths
-    // (N = 64 .. 512); other lengths return cudaErrorNotSupported for a batch.
+    // Members of a batch (sp.nmem > 1) run the MB instantiations, which exist for zr_size lengths (batches need the
+    // register z kernel, and gnss_batch_supported wants x and y of its lengths); other lengths return
+    // cudaErrorNotSupported for a batch.
     static cudaError_t pass(int sign, const PassPtrs<T> &P, const PassSpec &sp, const void *tw, int nsm,
                             cudaStream_t s, int pvariant, unsigned *err) {
         const bool mb = sp.nmem > 1;
@@ -84,9 +85,14 @@ template <typename T, int N> struct PassLaunch {
                 const long long nitems =
                     (long long)sp.nmem * sp.nin * (sp.list ? sp.nlist : sp.outer.count() * sd.ncolblk);
                 static std::atomic<int> per_sd[8];
-                auto kern = sign < 0 ? (mb ? k_passd<T, N, -1, false, true> : k_passd<T, N, -1>)
-                            : gen    ? (mb ? k_passd<T, N, +1, true, true> : k_passd<T, N, +1, true>)
-                                     : (mb ? k_passd<T, N, +1, false, true> : k_passd<T, N, +1>);
+                auto kern = sign < 0 ? k_passd<T, N, -1> : gen ? k_passd<T, N, +1, true> : k_passd<T, N, +1>;
+                if constexpr (zr_size(N)) {
+                    if (mb) kern = sign < 0 ? k_passd<T, N, -1, false, true>
+                                   : gen    ? k_passd<T, N, +1, true, true>
+                                            : k_passd<T, N, +1, false, true>;
+                } else if (mb) {
+                    return cudaErrorNotSupported;
+                }
                 return launch_persistent(kern, per_sd[ci + (gen ? 4 : 0)], C::NT, C::SMEM, nsm,
                                          nitems, s, P, sd, tw);
             }

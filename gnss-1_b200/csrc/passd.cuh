@@ -46,8 +46,7 @@ template <typename T, int N> struct PDCfg {
     static constexpr int NB = U * W;                         // columns per tile
     static constexpr int TPC = N == 48 ? 8 : N / 8;   // threads per column element
     static constexpr int NT = U * TPC;
-    static constexpr int BUFS = 2;
-    static constexpr int SMEM = BUFS * N * U * 16 + N * 16 + N * 8;   // tiles, twiddles, row wavenumbers
+    static constexpr int SMEM = 2 * N * U * 16 + N * 16 + N * 8;   // two tiles, twiddles, row wavenumbers
     // threads per SM the registers are sized for: 80 each, and 96 where 80 spill and few tiles make up for it (48^3
     // FP32 transform 16.5 -> 14.5 us, FP64 step 41.5 -> 37.3; 64^3 FP64 step 41.1 -> 38.7; 64 x 512 x 512 unchanged)
     static constexpr int THREADS = N == 48 || (N == 64 && W == 1) ? 640 : 768;
@@ -128,7 +127,7 @@ k_passd(const __grid_constant__ PassPtrs<T> Pp, const __grid_constant__ PassSpec
     constexpr int LAST = pd_stages(N) - 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     E *X = reinterpret_cast<E *>(smem_raw);
-    E *tw = X + C::BUFS * TILE;
+    E *tw = X + 2 * TILE;
     P *krow = reinterpret_cast<P *>(tw + N);
     const int tid = threadIdx.x, u = tid % U, t = tid / U;
     const bool own = M0 == TPC || t < M0;   // this thread has rows of stage 0
@@ -248,7 +247,6 @@ k_passd(const __grid_constant__ PassPtrs<T> Pp, const __grid_constant__ PassSpec
         cp_async_commit();
         cp_async_wait<1>();
         E *in = X + buf * TILE;
-        E *wk = C::BUFS == 3 ? X + 2 * TILE : in;
         E v[8];
         if (own) {
             const int mul = sp.vmul[cur.fi][var];
@@ -272,40 +270,31 @@ k_passd(const __grid_constant__ PassPtrs<T> Pp, const __grid_constant__ PassSpec
                     const P kr = krow[t + r * M0];
                     v[r] = E{pneg(kr * v[r].y), kr * v[r].x};
                 }
-            } else if (GEN && mul != V_ONE) {
+            } else if (GEN && mul != V_ONE) {   // V_LAP
                 const int c = cur.cb * NB + u * W;
                 const double ko = sp.n_out ? wavenum(sp.outer.expand(cur.oc), sp.n_out, sp.dk_out) : 0.0;
                 const double k0 = wavenum(c, sp.n_col, sp.dk_col), k1 = wavenum(c + 1, sp.n_col, sp.dk_col);
 #pragma unroll
                 for (int r = 0; r < 8; ++r) {
-                    if (mul == V_LAP) {
-                        const double kr = wavenum(t + r * M0, sp.n_row, sp.dk_row);
-                        P k2;
-                        if constexpr (W == 1) k2 = -ksq3(kr, ko, k0);
-                        else k2 = f2((float)-ksq3(kr, ko, k0), (float)-ksq3(kr, ko, k1));
-                        v[r] = E{k2 * v[r].x, k2 * v[r].y};
-                    } else {   // V_IK_OUT, V_IK_COL
-                        P kk;
-                        if constexpr (W == 1) kk = mul == V_IK_OUT ? ko : k0;
-                        else kk = mul == V_IK_OUT ? f2((float)ko, (float)ko) : f2((float)k0, (float)k1);
-                        v[r] = E{pneg(kk * v[r].y), kk * v[r].x};
-                    }
+                    const double kr = wavenum(t + r * M0, sp.n_row, sp.dk_row);
+                    P k2;
+                    if constexpr (W == 1) k2 = -ksq3(kr, ko, k0);
+                    else k2 = f2((float)-ksq3(kr, ko, k0), (float)-ksq3(kr, ko, k1));
+                    v[r] = E{k2 * v[r].x, k2 * v[r].y};
                 }
             }
             PDft<8, SIGN>::run(v);
         }
-        if constexpr (C::BUFS == 2) __syncthreads();
+        __syncthreads();
         if (own) {
 #pragma unroll
-            for (int r = 0; r < 8; ++r) wk[(t * 8 + r) * U + u] = v[r];
+            for (int r = 0; r < 8; ++r) in[(t * 8 + r) * U + u] = v[r];
         }
         __syncthreads();
-        const E *last = wk;
         if constexpr (LAST == 2) {
-            pd_stage<T, N, 1, SIGN, C::BUFS == 2>(
-                t, tw, [&](int row) -> E { return wk[row * U + u]; }, [&](int, int row, E e) { in[row * U + u] = e; });
+            pd_stage<T, N, 1, SIGN, true>(
+                t, tw, [&](int row) -> E { return in[row * U + u]; }, [&](int, int row, E e) { in[row * U + u] = e; });
             __syncthreads();
-            last = in;
         }
         // the tile after the next: looked up here, used in the next round
         Item nn = nxt;
@@ -335,7 +324,7 @@ k_passd(const __grid_constant__ PassPtrs<T> Pp, const __grid_constant__ PassSpec
         };
         const unsigned sm = left > 0 ? km & pd_rows<N>(t, tile_b) : 0u;
         pd_stage<T, N, LAST, SIGN, false>(
-            t, tw, [&](int row) -> E { return last[row * U + u]; },
+            t, tw, [&](int row) -> E { return in[row * U + u]; },
             [&](int i, int row, E e) {
                 if constexpr (C::OWN_LAST) {   // row t + i M0
                     if ((sm >> i) & 1u) put((i < 4 ? dlo : dhi) + i * (M0 * drow), e);
@@ -346,7 +335,7 @@ k_passd(const __grid_constant__ PassPtrs<T> Pp, const __grid_constant__ PassSpec
                 }
             });
         if (!go) break;
-        if constexpr (!C::OWN_LAST || (LAST == 1 && C::BUFS == 3)) __syncthreads();   // the tiles are free
+        if constexpr (!C::OWN_LAST) __syncthreads();   // the tiles are free
         if (more) {
             ++var;
         } else {

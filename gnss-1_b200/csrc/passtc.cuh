@@ -197,7 +197,6 @@ k_passtc(const __grid_constant__ PassPtrs<float> P, const __grid_constant__ Pass
         constexpr int MUL = decltype(mulc)::value;
         const int dmax = sp.mask ? dmax_s[pc] : N;
         const double kcd = wavenum(c0 + pc, sp.n_col, sp.dk_col);
-        const float kk = MUL == V_IK_OUT ? (float)k_out : (float)kcd;
         const float dkr = (float)sp.dk_row;
 #pragma unroll
         for (int it = 0; it < NIT; ++it) {
@@ -211,8 +210,6 @@ k_passtc(const __grid_constant__ PassPtrs<float> P, const __grid_constant__ Pass
                 if constexpr (MUL == V_IK_ROW) {
                     const float kr = dkr * (float)(row < N / 2 ? row : row - N);
                     x = V{-kr * x.y, kr * x.x};
-                } else if constexpr (MUL == V_IK_OUT || MUL == V_IK_COL) {
-                    x = V{-kk * x.y, kk * x.x};
                 } else if constexpr (MUL == V_LAP) {
                     const float k2 = (float)ksq3(wavenum(row, N, sp.dk_row), k_out, kcd);
                     x = V{-k2 * x.x, -k2 * x.y};
@@ -231,8 +228,6 @@ k_passtc(const __grid_constant__ PassPtrs<float> P, const __grid_constant__ Pass
     auto build_a1 = [&](int mul, int c0, double k_out) {
         switch (mul) {
             case V_IK_ROW: build_a1_mul(std::integral_constant<int, V_IK_ROW>{}, c0, k_out); break;
-            case V_IK_OUT: build_a1_mul(std::integral_constant<int, V_IK_OUT>{}, c0, k_out); break;
-            case V_IK_COL: build_a1_mul(std::integral_constant<int, V_IK_COL>{}, c0, k_out); break;
             case V_LAP: build_a1_mul(std::integral_constant<int, V_LAP>{}, c0, k_out); break;
             default: build_a1_mul(std::integral_constant<int, V_ONE>{}, c0, k_out); break;
         }

@@ -4,10 +4,6 @@
 #include "launch.cuh"
 #include "zreg.cuh"
 
-// GNSS_VARIANT_AUTO takes a register z kernel at every length one serves
-// (measured on ensembles of 16 x 64^3 .. 2 x 192^3 and single jets at 256^3, 512^3)
-__host__ __device__ constexpr bool zr_auto_z(int n) { return zr_size(n); }
-
 template <typename T, int N> struct ZLaunch {
     template <int NPH, int NRAW, bool PP>
     static cudaError_t zphys_k(const FieldSet<T> &f, const ZRecipeSet &zr, int nout, long long nlines, int ncp,
@@ -118,16 +114,16 @@ template <typename T, int N> struct ZLaunch {
             return false;
         }
     }
-    // the z kernel a variant option selects: GNSS_VARIANT_WARPSPEC and _REGISTER both name k_zpipe (the first where
-    // zws_fits; AUTO reports it so in FP64), _STAGED k_zphys
+    // the z kernel a variant option selects: GNSS_VARIANT_WARPSPEC and _REGISTER both name the register kernel (k_zpipe
+    // in FP32, k_zws in FP64; the first name where zws_fits, and AUTO answers so in FP64), _STAGED k_zphys
     static int zkernel(int zvariant, int nph, int nraw, int nout, int ncp) {
         const bool ws = zvariant == GNSS_VARIANT_WARPSPEC || (zvariant == GNSS_VARIANT_AUTO && sizeof(T) == 8);
         if (ws && zws_fits(nph, nraw, nout, ncp)) return GNSS_VARIANT_WARPSPEC;
-        const bool reg = zvariant == GNSS_VARIANT_REGISTER || zvariant == GNSS_VARIANT_WARPSPEC ||
-                         (zvariant == GNSS_VARIANT_AUTO && zr_auto_z(N));
-        return reg && zreg_fits(nph, nraw, ncp) ? GNSS_VARIANT_REGISTER : GNSS_VARIANT_STAGED;
+        // AUTO takes a register kernel at every length one serves (measured on ensembles of 16 x 64^3 .. 2 x 192^3 and
+        // single jets at 256^3, 512^3)
+        return zvariant != GNSS_VARIANT_STAGED && zreg_fits(nph, nraw, ncp) ? GNSS_VARIANT_REGISTER : GNSS_VARIANT_STAGED;
     }
-    // diag != nullptr: k_zpipe with the fused vorticity sums (cudaErrorNotSupported where it does not exist)
+    // diag != nullptr: the register kernel with the fused vorticity sums (cudaErrorNotSupported where none exists)
     static cudaError_t zphys(const FieldSet<T> &f, const ZRecipeSet &zr, int nph, int nraw, int nout,
                              long long nlines, int ncp, int nkz, T scale, T alpha, double dkz, const void *tw,
                              unsigned *err, int nsm, cudaStream_t s, int zvariant, double *diag = nullptr,

@@ -109,7 +109,7 @@ template <typename T, int N> struct ZRCfg {
     static constexpr bool POW2 = E == 16 && sizeof(T) == 8;
     static constexpr int ROWS = SHFL ? E : POW2 ? 4 : (E == 16 ? 6 : 4);
     // line padding.  Transpose scheme: a warp's stores of a transform's
-    // output (zr_out_index: lane groups j = lane % G at E^2 sigma(j) apart,
+    // output (zr_fft: lane groups j = lane % G at E^2 sigma(j) apart,
     // lanes of a group on consecutive entries) take one wavefront per 128
     // bytes when every group starts on its own bank range, so PADP entries
     // follow every PADB = E^2: 64 bytes for E = 16 (two groups), 32 for E = 8
@@ -376,17 +376,8 @@ __device__ __forceinline__ void zr_fft(int lane, V2<T> *x, V2<T> *scr, const V2<
     }
 }
 
-// Line index held in x[q] after zr_fft.
-template <typename T, int N> __device__ __forceinline__ int zr_out_index(int lane, int q) {
-    using Z = ZRCfg<T, N>;
-    if constexpr (Z::SHFL)
-        return q + Z::E * (int)(__brev((unsigned)lane) >> 27);
-    else
-        return lane / Z::G + Z::E * q + Z::E * Z::E * zr_sigma<Z::G>(lane % Z::G);
-}
-
-// The reverse of zr_fft: on entry x[q] is element zr_out_index(lane, q), on
-// return x[m] is element lane + 32 m of the length-N DFT.  With input index
+// The reverse of zr_fft: on entry x[q] is the element that zr_fft returns there,
+// on return x[m] is element lane + 32 m of the length-N DFT.  With input index
 // n = k1 + E k2 and output index k = l + 32 m, W_N^(n k) = W_E^(k1 m)
 // W_N^(k1 l) W_32^(k2 l): a 32-point DFT over k2 (k2 = q + E s, l = G l' + j:
 // a G-point DFT across the lanes, W_32^(q j), an E-point DFT over q), the
@@ -562,9 +553,9 @@ __device__ __forceinline__ void zl_unpack(int lane, const V2<T> *x, V2<T> *d, in
 }
 
 // Physical lines and their products.  A warp leaves a physical line in shared
-// memory where its transform ends: element zr_out_index(lane, q) at
-// zl_base(lane) + q zl_stride() of the line (PADB / PADC padding: no bank
-// conflicts), and the forward warps read the products' factors at the same
+// memory where its transform ends: x[q] of zr_fft at zl_base(lane) + q
+// zl_stride() of the line, which is its element's place (PADB / PADC padding:
+// no bank conflicts), and the forward warps read the products' factors at the same
 // places.  Quantities: 0 u, 1 v, 2 w, 3 w1, 4 w2, 5 w3, 6 sx, 7 sy, 8 sz,
 // [9 cx, 10 cy, 11 cz], [12 c, 13 lap s].
 template <typename T, int N> __device__ __forceinline__ int zl_base(int lane) {
