@@ -110,10 +110,27 @@ static int device_of_reuse() {
     return 0;
 }
 
+// A state of several MB is copied in and out in parts, byte for byte.
+static int large_state() {
+    gnss_config c = config(96);
+    c.nz = 64;   // 96 x 96 x 33 x 4 x 8 bytes, 9.7 MB
+    std::vector<char> st = state_of(c), out(st.size(), 0);
+    for (size_t i = 0; i < st.size(); ++i) st[i] = (char)(i * 31 + (i >> 13));
+    gnss_server *s = server(2);
+    long long id = 0;
+    EXPECT(gnss_server_submit(s, &c, st.data(), 3, &id) == GNSS_OK);
+    EXPECT(gnss_server_wait(s, id, 10.0) == GNSS_OK);
+    EXPECT(gnss_server_result(s, id, out.data(), nullptr, nullptr) == GNSS_OK);
+    EXPECT(st == out);
+    EXPECT(gnss_server_destroy(s) == GNSS_OK);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string name = argc > 1 ? argv[1] : "";
     if (name == "failed_request") return failed_request();
     if (name == "idle_contexts") return idle_contexts();
     if (name == "device_of_reuse") return device_of_reuse();
+    if (name == "large_state") return large_state();
     return 2;
 }

@@ -43,7 +43,7 @@ def server(tmp_path_factory):
                     CSRC / "batch.cpp")
 
 
-@pytest.mark.parametrize("scenario", ["failed_request", "idle_contexts", "device_of_reuse"])
+@pytest.mark.parametrize("scenario", ["failed_request", "idle_contexts", "device_of_reuse", "large_state"])
 def test_server(server, scenario):
     r = _run(server, scenario)
     assert r.returncode == 0, r.stdout + r.stderr
