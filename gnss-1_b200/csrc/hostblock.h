@@ -59,7 +59,9 @@ SphereTables sphere_tables(SphereAxis x, SphereAxis y, SphereAxis z, double kmax
 // Copies pageable host memory to the device and waits until it is there.
 // cudaMemcpy from pageable memory may return once the data lies in its staging
 // buffer, and work on a non-blocking stream does not wait for the stream that
-// carries the rest of the copy.
+// carries the rest of the copy.  (That stream alone is waited for: a device
+// synchronisation would break a capture on another thread, as the server's
+// scheduler makes them.)
 inline cudaError_t upload_and_wait(void *dst, const void *src, size_t bytes) {
     const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
     return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
