@@ -11,14 +11,14 @@
 // to global memory.  Eight elements per thread keep it at 80 registers, 24
 // warps per SM (16 at N = 512, whose two tiles fill an SM's shared memory).
 //   What bounds it: instruction issue and shared-memory wavefronts (ncu, 512
-//   rows: LSU wavefronts 54-59% FP64, 53-56% FP32, issue 40 / 45%), so what is fixed
+//   rows: LSU wavefronts 60-65% FP64, 53-56% FP32, issue 38 / 45%), so what is fixed
 //   for the launch stays out of the loop: the rows a thread reads and stores
 //   as bit masks, work items advanced by the grid size instead of divided,
 //   two base pointers (lower and upper half of the rows: the gap of a compact
 //   axis lies between them) plus a uniform stride.
 //   Measured against the register kernel it replaced (one warp per column, 8
 //   FP64 / 16 FP32 warps per SM), the four passes of a step: 512^3 FP64 with
-//   two scalars 7.98 -> 6.66 ms, 512^3 FP32 4.09 -> 2.95, 256^3 FP32 0.71 ->
+//   two scalars 7.98 -> 6.48 ms, 512^3 FP32 4.09 -> 2.99, 256^3 FP32 0.71 ->
 //   0.36, 192^3 FP32 0.36 -> 0.18 ms.
 //   The dealiasing sphere: rows outside it are not read, tiles outside it are
 //   not visited (21% of the x passes' tiles), and rows no later stage reads

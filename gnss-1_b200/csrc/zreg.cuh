@@ -738,8 +738,8 @@ template <typename T, int N, int NPH> struct ZPipe {   // FP32
 // sets bit 0 of *err and the block stops.  With DIAG the block writes one row
 // of ZR_VORT_SUMS vorticity sums over its points to diag[blockIdx.x], for the
 // statistics of the state the step starts from.
-//   What bounds it (ncu, 512-point lines): issue 58%, shared-memory wavefronts
-// 59%.  Against a block of NPH warps of which NOUT run the forward transforms
+//   What bounds it (ncu, 512-point lines): issue 57%, shared-memory wavefronts
+// 63%.  Against a block of NPH warps of which NOUT run the forward transforms
 // after a products phase (two more barriers, NPH - NOUT warps idle): 512^3 one
 // scalar 2.52 -> 2.08 ms, 256^3 one scalar 0.380 -> 0.314, two scalars 0.725 ->
 // 0.402 ms (there one block per SM before).  In FP64 the forward warps' reads
@@ -919,7 +919,7 @@ template <typename T, int N, int NPH> struct ZWs {
 // forms the products of p into the forward warps' lines.  The raw lines of the
 // next pair are requested as soon as every inverse warp has packed (named
 // barrier 1).
-//   What bounds it (ncu, 512-point lines): shared-memory wavefronts 59%, the
+//   What bounds it (ncu, 512-point lines): shared-memory wavefronts 65%, the
 // FP64 pipe 42%, with one block of 13 or 17 warps per SM.  Reading each raw
 // mode once (the mirrored half by shuffle), transforming the products in the
 // reversed flow graph and storing them from registers took 512^3 from 5.53 to
